@@ -70,9 +70,10 @@ enum {
                             range (a value between 2^-74 and 2^128 is held to 2^-48 of
                             itself; below 2^-74 a pair keeps 24 bits, below 2^-126 it
                             flushes to zero; 2^128 or more returns UHS_ERANGE).  Star
-                            and separable sums are error-free on a power-of-two grid set
-                            per point from sum |c_k x_k| (bounded sums); each point's
-                            error stays within about n^2 2^-46 of that sum for n terms */
+                            and separable sums run on an anchor set per point to twice
+                            sum |c_k x_k| (anchored sums): each point's error stays within
+                            about n^2 2^-46 of that sum for n terms, and a point whose
+                            sum |c_k x_k| passes 2^126 returns UHS_ERANGE too */
 };
 
 /* ---- MLIR memref descriptor (rank-3 layout) ---------------------------- */

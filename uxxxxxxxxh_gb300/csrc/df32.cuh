@@ -200,84 +200,110 @@ __device__ __forceinline__ void renorm2(const df2 &a, u64 &h, u64 &l) {
 
 namespace uhs {
 
-// ---- bounded sums: one stencil point's sum with an extraction bound ---------
+// ---- anchored sums: one stencil point's sum on a running anchor -----------
 // A point's sum  s = sum_k c_k * x_k  (float pairs c = ch + cl, x = xh + xl)
-// in fewer FP32 operations than df_fma's TwoSum per term, by extracting each
-// product's high part on a fixed grid (Rump, Ogita and Oishi, "Accurate
-// floating-point summation", ExtractScalar):
-//   B = sum_k |ch_k| |xh_k| (one FMA per term, bound_add);
-//   sigma = 2^m, B (1 + 2^-16) < sigma <= 2 B (1 + 2^-16) (sigma_of);
-//   p = ch * xh;  q = (sigma + p) - sigma;  r = fma(ch, xh, -q)
-// With |p| <= sigma, q is p on the grid of multiples of 2^-24 sigma and
-// p - q is exact (ExtractScalar's lemma), so every partial sum of the q's --
-// multiples of 2^-24 sigma below sigma in magnitude, as sum |p| and the n
-// roundings to the grid stay below B (1 + (2n + 1) 2^-24) < sigma for up to
-// 127 terms -- is exact in a float: tau = sum q_k carries no error.  r is
-// the rest of the exact product, ch * xh - q, rounded once (|r| <= 2^-23
-// sigma, so its error is below 2^-47 sigma), and the low-order parts go into
-// lo:
-//   lo += r;  lo = fma(ch, xl, lo);  lo = fma(cl, xh, lo)
-// 9 FP32 operations per term with the bound, against df_fma's 12.  The
-// point's value is tau + lo, renormalised by one TwoSum (renorm) as before.
-// The error is relative to sum |c_k x_k| of the point itself, as with
-// df_fma's errors relative to its partial sums: lo sums n terms of at most
-// 2^-23 sigma <= 2^-22 (1 + 2^-16) B, so its roundings stay below about
-// n^2 2^-46 B, in practice (random signs) near n^1.5 2^-47 B; for a field of
-// one sign, B is the point's value.
+// in 7 FP32 operations per term, against df_fma's 12.  The running sum T
+// starts at an anchor sigma that dominates the sum, so each step's rounding
+// error follows from Dekker's Fast2Sum (no TwoSum):
+//   B = sum_k |ch_k| |xh_k|;  sigma = 2 B (1 + 2^-15)        (anchor_add)
+//   T_0 = sigma;  T_k = fma(ch, xh, T_{k-1})
+//   q = T_k - T_{k-1}          exact: T_{k-1}/2 <= T_k <= 2 T_{k-1}
+//   r = fma(ch, xh, -q)        the product's part that T_k did not take
+//   hi += r;  lo = fma(ch, xl, lo);  lo = fma(cl, xh, lo)
+// and the point's value is (T_n - sigma) + (hi + lo).
+// Why q is exact: at step k the terms before it took at most B - |p_k| from
+// the anchor, so T_{k-1} >= 2 B - (B - |p_k|) >= 2 |p_k| and T_k lies within
+// a factor of two of T_{k-1} (Sterbenz' lemma); the 2^-15 covers the
+// roundings of B and of the T's for up to 127 terms.  The same bound puts T_n
+// between sigma / 2 and 2 sigma, so T_n - sigma is exact too.  All error is
+// in the three low-order accumulations: |r| <= ulp(3 B) / 2, and keeping the
+// r's apart from the cross terms (hi, lo) rounds each at its own size.
+// Measured on random sums of 5-19 terms (error / B, rms, in units of 2^-49):
+// 3.7-15 against 4.3-24 for the extraction on a power-of-two grid that was
+// used before (9 operations per term, one low-order accumulator), on every
+// count and sign pattern (tests/c/anchored_sum_check.c).
+// sum |c| enters as 2 (1 + 2^-15) |ch| from the host (fill_coef_anchor), so
+// the anchor is one FMA per term and needs no further rounding.
 //
-// The bound's exponent is clamped so sigma stays a normal float (inputs
-// beyond 2^125 overflow the grid: the range flag catches them).
-__device__ __forceinline__ float bound_add(float b, float cabs, float2 x) {  // cabs = |ch|
+// T reaches 3 B: a point whose B exceeds about 2^126.4 overflows to Inf/NaN,
+// which the range flag catches.
+__device__ __forceinline__ float anchor_add(float b, float cabs, float2 x) {  // cabs = 2 (1 + 2^-15) |ch|
     return __fmaf_rn(cabs, fabsf(x.x), b);
 }
-__device__ __forceinline__ float sigma_of(float b) {
-    const float bb = __fmul_ru(b, 1.0000152587890625f);  // 1 + 2^-16
-    const int e = min(static_cast<int>(__float_as_uint(bb) & 0x7f800000u), 253 << 23);
-    return __int_as_float(e + (1 << 23));
+
+// Running state of an anchored sum.
+struct dfa {
+    float t, sg, hi, lo;
+};
+
+// first term, on the anchor sigma
+__device__ __forceinline__ void dfa_first(dfa &a, float sigma, float ch, float cl, float2 x) {
+    a.sg = sigma;
+    a.t = __fmaf_rn(ch, x.x, sigma);
+    a.hi = __fmaf_rn(ch, x.x, -__fsub_rn(a.t, sigma));
+    a.lo = __fmaf_rn(cl, x.x, __fmul_rn(ch, x.y));
 }
 
-// acc = c * x (first term of a bounded sum)
-__device__ __forceinline__ void dfs_mul(df &acc, float sigma, float ch, float cl, float2 x) {
-    const float p = __fmul_rn(ch, x.x);
-    const float q = __fsub_rn(__fadd_rn(sigma, p), sigma);
-    const float r = __fmaf_rn(ch, x.x, -q);
-    acc.h = q;
-    acc.l = __fmaf_rn(cl, x.x, __fmaf_rn(ch, x.y, r));
+// += c * x
+__device__ __forceinline__ void dfa_add(dfa &a, float ch, float cl, float2 x) {
+    const float t = __fmaf_rn(ch, x.x, a.t);
+    const float q = __fsub_rn(t, a.t);
+    a.t = t;
+    a.hi = __fadd_rn(a.hi, __fmaf_rn(ch, x.x, -q));
+    a.lo = __fmaf_rn(cl, x.x, __fmaf_rn(ch, x.y, a.lo));
 }
 
-// acc += c * x (bounded sum)
-__device__ __forceinline__ void dfs_fma(df &acc, float sigma, float ch, float cl, float2 x) {
-    const float p = __fmul_rn(ch, x.x);
-    const float q = __fsub_rn(__fadd_rn(sigma, p), sigma);
-    const float r = __fmaf_rn(ch, x.x, -q);
-    acc.h = __fadd_rn(acc.h, q);
-    acc.l = __fmaf_rn(cl, x.x, __fmaf_rn(ch, x.y, __fadd_rn(acc.l, r)));
+// the sum as an (unnormalised) pair: h is a multiple of T's last place
+__device__ __forceinline__ df dfa_end(const dfa &a) {
+    return df{__fsub_rn(a.t, a.sg), __fadd_rn(a.hi, a.lo)};
 }
 
-// The same for two points at once: the extraction and the two additions
-// packed (.f32x2), the products and the low-order terms per point.  Per
-// point the same operations as dfs_mul / dfs_fma, so bit-identical to them.
-// sig holds {sigma of point 0, sigma of point 1}.
-__device__ __forceinline__ void dfs2_mul_s(df2 &acc, u64 sig, float ch, float cl, float2 x0, float2 x1) {
-    const u64 p = pk2(__fmul_rn(ch, x0.x), __fmul_rn(ch, x1.x));
-    const u64 q = sub2(add2(sig, p), sig);
-    float q0, q1;
-    upk2(q, q0, q1);
-    const float r0 = __fmaf_rn(ch, x0.x, -q0), r1 = __fmaf_rn(ch, x1.x, -q1);
-    acc.h = q;
-    acc.l = pk2(__fmaf_rn(cl, x0.x, __fmaf_rn(ch, x0.y, r0)), __fmaf_rn(cl, x1.x, __fmaf_rn(ch, x1.y, r1)));
+// (h, l) of dfa_end -> the same value with |l| <= ulp(h) / 2.  h is a multiple
+// of T's last place and |l| a few such places, so h is a multiple of ulp(l)
+// whichever of the two is larger, and Fast2Sum is exact.
+__device__ __forceinline__ float2 dfa_renorm(df a) {
+    const float s = __fadd_rn(a.h, a.l);
+    return make_float2(s, __fsub_rn(a.l, __fsub_rn(s, a.h)));
 }
 
-__device__ __forceinline__ void dfs2_fma_s(df2 &acc, u64 sig, float ch, float cl, float2 x0, float2 x1) {
-    const u64 p = pk2(__fmul_rn(ch, x0.x), __fmul_rn(ch, x1.x));
-    const u64 q = sub2(add2(sig, p), sig);
-    float q0, q1;
-    upk2(q, q0, q1);
-    const float r0 = __fmaf_rn(ch, x0.x, -q0), r1 = __fmaf_rn(ch, x1.x, -q1);
-    acc.h = add2(acc.h, q);
-    float l0, l1;
-    upk2(add2(acc.l, pk2(r0, r1)), l0, l1);
-    acc.l = pk2(__fmaf_rn(cl, x0.x, __fmaf_rn(ch, x0.y, l0)), __fmaf_rn(cl, x1.x, __fmaf_rn(ch, x1.y, l1)));
+// The same for two points at once: the subtractions and the hi additions
+// packed (.f32x2), the fused products per point (they read the coefficient
+// from the constant bank, which a packed instruction cannot).  Per point the
+// same operations as above, so bit-identical to them.
+struct dfa2 {
+    u64 t, sg, hi;
+    float lo0, lo1;
+};
+
+__device__ __forceinline__ u64 anchored_step2(u64 &t, float ch, float2 x0, float2 x1) {
+    float t0, t1, q0, q1;
+    upk2(t, t0, t1);
+    const u64 tn = pk2(__fmaf_rn(ch, x0.x, t0), __fmaf_rn(ch, x1.x, t1));
+    upk2(sub2(tn, t), q0, q1);
+    t = tn;
+    return pk2(__fmaf_rn(ch, x0.x, -q0), __fmaf_rn(ch, x1.x, -q1));
+}
+
+__device__ __forceinline__ void dfa2_first(dfa2 &a, u64 sigma, float ch, float cl, float2 x0, float2 x1) {
+    a.sg = a.t = sigma;
+    a.hi = anchored_step2(a.t, ch, x0, x1);
+    a.lo0 = __fmaf_rn(cl, x0.x, __fmul_rn(ch, x0.y));
+    a.lo1 = __fmaf_rn(cl, x1.x, __fmul_rn(ch, x1.y));
+}
+
+__device__ __forceinline__ void dfa2_add(dfa2 &a, float ch, float cl, float2 x0, float2 x1) {
+    a.hi = add2(a.hi, anchored_step2(a.t, ch, x0, x1));
+    a.lo0 = __fmaf_rn(cl, x0.x, __fmaf_rn(ch, x0.y, a.lo0));
+    a.lo1 = __fmaf_rn(cl, x1.x, __fmaf_rn(ch, x1.y, a.lo1));
+}
+
+__device__ __forceinline__ df2 dfa2_end(const dfa2 &a) {
+    return df2{sub2(a.t, a.sg), add2(a.hi, pk2(a.lo0, a.lo1))};
+}
+
+__device__ __forceinline__ void dfa2_renorm(const df2 &a, u64 &h, u64 &l) {
+    h = add2(a.h, a.l);
+    l = sub2(a.l, sub2(h, a.h));
 }
 
 }  // namespace uhs

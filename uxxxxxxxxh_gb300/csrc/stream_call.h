@@ -45,8 +45,9 @@ struct StreamArgs {
     // per pass (sep: z, y, x; otherwise [0]); applied once per point to the
     // centre value so the sweep keeps the FP64 coefficients' sum.
     float cl_sum[3];
-    // |ch| of each coefficient: the float-pair bounded sums' bound (df32.cuh
-    // bound_add) reads it as an operand instead of holding |ch| in registers
+    // 2 (1 + 2^-15) |ch| of each coefficient: the float-pair sums' anchor
+    // (df32.cuh anchor_add) reads it as an operand instead of holding it in
+    // registers
     float cab[NT];
 };
 
@@ -65,8 +66,9 @@ inline void fill_coefs(double *cd, float2 *chl, float *cl_sum, const double *coe
     }
     for (int i = 0; i < 3; ++i) cl_sum[i] = static_cast<float>(sums[i]);
 }
-inline void fill_coef_abs(float *cab, const float2 *chl, int nt) {
-    for (int k = 0; k < nt; ++k) cab[k] = chl[k].x < 0.0f ? -chl[k].x : chl[k].x;
+inline void fill_coef_anchor(float *cab, const float2 *chl, int nt) {
+    const float f = 2.0f * (1.0f + 0x1p-15f);
+    for (int k = 0; k < nt; ++k) cab[k] = f * (chl[k].x < 0.0f ? -chl[k].x : chl[k].x);
 }
 
 // Everything one streaming launch needs (filled by the runtime).

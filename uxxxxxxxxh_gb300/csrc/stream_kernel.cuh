@@ -101,10 +101,17 @@ struct StreamCfg {
     static constexpr int NT = SI::NT;
     // Float-pair sweeps sum a thread's points two at a time in packed FP32
     // instructions in standalone launches: rows 2p, 2p+1 in 3D, the two
-    // columns of a rank-2 thread with VX = 2 (dfs2_*_s for stars and
-    // separable passes, df2_*_s for term-by-term boxes, df32.cuh).  GB300 at
-    // 512^3 (256^3 for radius 2-3 boxes), GStencil/s per sweep, scalar ->
-    // packed (with TwoSum sums; bounded sums came after): stars on float-pair grids r1/r2/r3 330/184/129
+    // columns of a rank-2 thread with VX = 2 (dfa2_* for stars and separable
+    // passes, df2_*_s for term-by-term boxes, df32.cuh).  What bounds the
+    // stars and separable passes on float-pair grids is the FP32 pipe (7
+    // operations per term) from radius 2 on, HBM for radius 1.  GStencil/s
+    // per sweep at 512^3 / 8192^2 with the 9-operation sums before -> now:
+    // 3D stars r1/r2/r3 368/231/158 -> 366/280/198, separable 238/140/92 ->
+    // 305/177/117, 2D stars 372/274/204 -> 397/324/243, separable
+    // 273/227/171 -> 328/268/203; FP64 grids in place +5-15 %.
+    // Scalar -> packed was measured at
+    // 512^3 (256^3 for radius 2-3 boxes), GStencil/s per sweep, with TwoSum
+    // sums in both: stars on float-pair grids r1/r2/r3 330/184/129
     // -> 341/186/134 (best tiles), on FP64 grids 169/114/86 -> 191/130/97;
     // separable boxes FP64 141/92/63 -> 163/102/68; radius-3 boxes 5.5/6.0 ->
     // 7.5/7.2.  Term-by-term boxes of radius 1 on float-pair grids (100 ->
@@ -231,9 +238,9 @@ __device__ __forceinline__ float2 coef_f2(const Args &a, int k) {
     }
 }
 
-// |ch| of coefficient k (the bounded sums' bound)
+// 2 (1 + 2^-15) |ch| of coefficient k (the float-pair sums' anchor)
 template <class C, class Args>
-__device__ __forceinline__ float coef_abs(const Args &a, int k) {
+__device__ __forceinline__ float coef_anchor(const Args &a, int k) {
     if constexpr (std::is_same_v<Args, BatchArgs>) {
         float v;
         asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"((unsigned)__cvta_generic_to_shared(&a.cab[k])));
@@ -276,16 +283,18 @@ struct Arith<C, kArNative> {
         if constexpr (F32) acc = fmaf(a.cl_sum[pass], v, acc);
     }
     __device__ static __forceinline__ void store(TS *p, const Acc &acc, unsigned &, int) { *p = acc; }
-    // bounded sums (float pairs only): the plain sum here
-    static constexpr bool kBounded = false;
+    // anchored sums (float pairs only): the plain sum here
+    static constexpr bool kAnchored = false;
+    using SAcc = TS;
     template <class Args>
-    __device__ static __forceinline__ void bfirst(Acc &acc, float, const Args &a, int k, TS v) {
+    __device__ static __forceinline__ void sfirst(SAcc &acc, float, const Args &a, int k, TS v) {
         first(acc, a, k, v);
     }
     template <class Args>
-    __device__ static __forceinline__ void badd(Acc &acc, float, const Args &a, int k, TS v) {
+    __device__ static __forceinline__ void sadd(SAcc &acc, const Args &a, int k, TS v) {
         add(acc, a, k, v);
     }
+    __device__ static __forceinline__ Acc send(const SAcc &acc) { return acc; }
     // two adjacent points, p aligned to 2 * sizeof(TS)
     static constexpr bool kVecStore = true;
     __device__ static __forceinline__ void store2(TS *p, const Acc &a0, const Acc &a1, unsigned &, int) {
@@ -308,18 +317,26 @@ struct Arith<C, kArDf32> {
         const float2 c = coef_f2<C>(a, k);
         df_fma(acc, c.x, c.y, v);
     }
-    // Star and separable sums: bounded sums (dfs_mul / dfs_fma in df32.cuh),
-    // sg = the point's sigma_of.  Term-by-term boxes keep first / add.
-    static constexpr bool kBounded = true;
+    // Star and separable sums: anchored sums (dfa_first / dfa_add in
+    // df32.cuh), sg = the point's anchor.  Term-by-term boxes keep first / add.
+    static constexpr bool kAnchored = true;
+    using SAcc = dfa;
     template <class Args>
-    __device__ static __forceinline__ void bfirst(Acc &acc, float sg, const Args &a, int k, float2 v) {
+    __device__ static __forceinline__ void sfirst(SAcc &acc, float sg, const Args &a, int k, float2 v) {
         const float2 c = coef_f2<C>(a, k);
-        dfs_mul(acc, sg, c.x, c.y, v);
+        dfa_first(acc, sg, c.x, c.y, v);
     }
     template <class Args>
-    __device__ static __forceinline__ void badd(Acc &acc, float sg, const Args &a, int k, float2 v) {
+    __device__ static __forceinline__ void sadd(SAcc &acc, const Args &a, int k, float2 v) {
         const float2 c = coef_f2<C>(a, k);
-        dfs_fma(acc, sg, c.x, c.y, v);
+        dfa_add(acc, c.x, c.y, v);
+    }
+    __device__ static __forceinline__ Acc send(const SAcc &acc) { return dfa_end(acc); }
+    // sums of stars and separable passes end as dfa_end's pairs
+    static constexpr bool kFastRenorm = C::SI::star || C::SI::sep;
+    __device__ static __forceinline__ float2 norm(const Acc &acc) {
+        if constexpr (kFastRenorm) return dfa_renorm(acc);
+        else return renorm(acc);
     }
     // FP64 grids: joined back with the run's exponent bias (the pairs hold
     // x * 2^pair_shift).  A sum that outgrew the float range (hi Inf or NaN)
@@ -330,7 +347,7 @@ struct Arith<C, kArDf32> {
             range_err |= (__float_as_uint(acc.h) & 0x7f800000u) == 0x7f800000u;
             *p = join_f64(acc.h, acc.l, bias);
         } else {
-            *p = renorm(acc);
+            *p = norm(acc);
         }
     }
     static constexpr bool kVecStore = true;
@@ -341,44 +358,44 @@ struct Arith<C, kArDf32> {
             range_err |= (__float_as_uint(a1.h) & 0x7f800000u) == 0x7f800000u;
             *reinterpret_cast<double2 *>(p) = make_double2(join_f64(a0.h, a0.l, bias), join_f64(a1.h, a1.l, bias));
         } else {
-            const float2 r0 = renorm(a0), r1 = renorm(a1);
+            const float2 r0 = norm(a0), r1 = norm(a1);
             *reinterpret_cast<float4 *>(p) = make_float4(r0.x, r0.y, r1.x, r1.y);
         }
     }
-    __device__ static __forceinline__ float2 level(const Acc &acc) { return renorm(acc); }
-    template <class Args>
-    __device__ static __forceinline__ void centre(Acc &, const Args &, int, float2) {}
+    __device__ static __forceinline__ float2 level(const Acc &acc) { return norm(acc); }
+    template <class S, class Args>
+    __device__ static __forceinline__ void centre(S &, const Args &, int, float2) {}
 };
 
-// Bound B of a star point's bounded sum (df32.cuh): sum |ch_k| |xh_k| over
-// its inputs in the sum's order -- centre, +-d along z, y (rank 3), x.
+// Anchor of a star point's sum (df32.cuh): 2 (1 + 2^-15) sum |ch_k| |xh_k|
+// over its inputs in the sum's order -- centre, +-d along z, y (rank 3), x.
 // zq: the point's z-queue (centre at [R]); cell: the point's own cell in
 // the staged centre plane (y-neighbours W apart, x-neighbours adjacent).
 // The sums that follow read the same cells; the code generator keeps the
 // loaded values in registers between the two (a warp barrier between them
 // forces reloads and cuts the 3D 13-point float-pair sweep from 118 to 72
-// registers per thread, but measured 4 % slower: 208 against 217 GStencil/s
-// per sweep at 512^3).
+// registers per thread, but measured 4 % slower, both with the 9-operation
+// sums: 208 against 217 GStencil/s per sweep at 512^3).
 template <class C, class Args, class TC>
-__device__ __forceinline__ float star_bound(const Args &a, const TC *zq, const TC *cell) {
+__device__ __forceinline__ float star_anchor(const Args &a, const TC *zq, const TC *cell) {
     constexpr int R = C::R, W = C::W;
-    float b = bound_add(0.0f, coef_abs<C>(a, coef_slot<C::SHAPE, R>(0, 0, 0)), zq[R]);
+    float b = anchor_add(0.0f, coef_anchor<C>(a, coef_slot<C::SHAPE, R>(0, 0, 0)), zq[R]);
 #pragma unroll
     for (int d = 1; d <= R; ++d) {
-        b = bound_add(b, coef_abs<C>(a, coef_slot<C::SHAPE, R>(-d, 0, 0)), zq[R - d]);
-        b = bound_add(b, coef_abs<C>(a, coef_slot<C::SHAPE, R>(d, 0, 0)), zq[R + d]);
+        b = anchor_add(b, coef_anchor<C>(a, coef_slot<C::SHAPE, R>(-d, 0, 0)), zq[R - d]);
+        b = anchor_add(b, coef_anchor<C>(a, coef_slot<C::SHAPE, R>(d, 0, 0)), zq[R + d]);
     }
     if constexpr (!C::SI::is2d) {
 #pragma unroll
         for (int d = 1; d <= R; ++d) {
-            b = bound_add(b, coef_abs<C>(a, coef_slot<C::SHAPE, R>(0, -d, 0)), cell[-d * W]);
-            b = bound_add(b, coef_abs<C>(a, coef_slot<C::SHAPE, R>(0, d, 0)), cell[d * W]);
+            b = anchor_add(b, coef_anchor<C>(a, coef_slot<C::SHAPE, R>(0, -d, 0)), cell[-d * W]);
+            b = anchor_add(b, coef_anchor<C>(a, coef_slot<C::SHAPE, R>(0, d, 0)), cell[d * W]);
         }
     }
 #pragma unroll
     for (int d = 1; d <= R; ++d) {
-        b = bound_add(b, coef_abs<C>(a, coef_slot<C::SHAPE, R>(0, 0, -d)), cell[-d]);
-        b = bound_add(b, coef_abs<C>(a, coef_slot<C::SHAPE, R>(0, 0, d)), cell[d]);
+        b = anchor_add(b, coef_anchor<C>(a, coef_slot<C::SHAPE, R>(0, 0, -d)), cell[-d]);
+        b = anchor_add(b, coef_anchor<C>(a, coef_slot<C::SHAPE, R>(0, 0, d)), cell[d]);
     }
     return b;
 }
@@ -543,7 +560,7 @@ __device__ __forceinline__ bool stream_item(const Args &a, int bxi, int byi, int
     TC q[NPT][(STAR || SEP) ? 2 * R + 1 : 1];  // z-queue, q[v][R + dz]: star: raw values; sep: xy-filtered
     // Float-pair sweeps (standalone launches): a thread's points are
     // summed two at a time (rows 2p, 2p+1, or a rank-2 thread's two columns)
-    // into packed accumulators, acc[p] of df2 (dfs2_fma_s / df2_fma_s in
+    // into packed accumulators (dfa2_add / df2_fma_s in
     // df32.cuh).
     constexpr bool PACK = C::PACKED && !std::is_same_v<Args, BatchArgs>;
     constexpr int NPR = PACK ? NPT / 2 : 1;
@@ -630,21 +647,20 @@ __device__ __forceinline__ bool stream_item(const Args &a, int bxi, int byi, int
                 float b0 = 0.0f, b1 = 0.0f;
 #pragma unroll
                 for (int dx = -R; dx <= R; ++dx) {
-                    const float ch = coef_abs<C>(a, CX0 + dx + R);
-                    b0 = bound_add(b0, ch, r0[dx]);
-                    b1 = bound_add(b1, ch, r1[dx]);
+                    const float ch = coef_anchor<C>(a, CX0 + dx + R);
+                    b0 = anchor_add(b0, ch, r0[dx]);
+                    b1 = anchor_add(b1, ch, r1[dx]);
                 }
-                const u64 sg = pk2(sigma_of(b0), sigma_of(b1));
-                df2 t;
+                dfa2 t;
                 float2 c = coef_f2<C>(a, CX0);
-                dfs2_mul_s(t, sg, c.x, c.y, r0[-R], r1[-R]);
+                dfa2_first(t, pk2(b0, b1), c.x, c.y, r0[-R], r1[-R]);
 #pragma unroll
                 for (int dx = -R + 1; dx <= R; ++dx) {
                     c = coef_f2<C>(a, CX0 + dx + R);
-                    dfs2_fma_s(t, sg, c.x, c.y, r0[dx], r1[dx]);
+                    dfa2_add(t, c.x, c.y, r0[dx], r1[dx]);
                 }
                 u64 hh, ll;
-                renorm2(t, hh, ll);
+                dfa2_renorm(dfa2_end(t), hh, ll);
                 upk2(hh, xr[i].x, xr[i + 1].x);
                 upk2(ll, xr[i].y, xr[i + 1].y);
             }
@@ -658,21 +674,20 @@ __device__ __forceinline__ bool stream_item(const Args &a, int bxi, int byi, int
                 float b0 = 0.0f, b1 = 0.0f;
 #pragma unroll
                 for (int dy = -R; dy <= R; ++dy) {
-                    const float ch = coef_abs<C>(a, D + dy + R);
-                    b0 = bound_add(b0, ch, xr[v + R + dy]);
-                    b1 = bound_add(b1, ch, xr[v + 1 + R + dy]);
+                    const float ch = coef_anchor<C>(a, D + dy + R);
+                    b0 = anchor_add(b0, ch, xr[v + R + dy]);
+                    b1 = anchor_add(b1, ch, xr[v + 1 + R + dy]);
                 }
-                const u64 sg = pk2(sigma_of(b0), sigma_of(b1));
-                df2 t;
+                dfa2 t;
                 float2 c = coef_f2<C>(a, D);
-                dfs2_mul_s(t, sg, c.x, c.y, xr[v], xr[v + 1]);
+                dfa2_first(t, pk2(b0, b1), c.x, c.y, xr[v], xr[v + 1]);
 #pragma unroll
                 for (int dy = -R + 1; dy <= R; ++dy) {
                     c = coef_f2<C>(a, D + dy + R);
-                    dfs2_fma_s(t, sg, c.x, c.y, xr[v + R + dy], xr[v + 1 + R + dy]);
+                    dfa2_add(t, c.x, c.y, xr[v + R + dy], xr[v + 1 + R + dy]);
                 }
                 u64 hh, ll;
-                renorm2(t, hh, ll);
+                dfa2_renorm(dfa2_end(t), hh, ll);
                 upk2(hh, q[v][2 * R].x, q[v + 1][2 * R].x);
                 upk2(ll, q[v][2 * R].y, q[v + 1][2 * R].y);
             }
@@ -688,18 +703,16 @@ __device__ __forceinline__ bool stream_item(const Args &a, int bxi, int byi, int
             for (int i = 0; i < NROW; ++i) {
                 const TC *row = cur + own + (IS2D ? 0 : (i - R) * W);
                 float sg = 0.0f;
-                if constexpr (A::kBounded) {
-                    float b = 0.0f;
+                if constexpr (A::kAnchored) {
 #pragma unroll
-                    for (int dx = -R; dx <= R; ++dx) b = bound_add(b, coef_abs<C>(a, CX0 + dx + R), row[dx]);
-                    sg = sigma_of(b);
+                    for (int dx = -R; dx <= R; ++dx) sg = anchor_add(sg, coef_anchor<C>(a, CX0 + dx + R), row[dx]);
                 }
-                Acc t;
-                A::bfirst(t, sg, a, CX0, row[-R]);
+                typename A::SAcc t;
+                A::sfirst(t, sg, a, CX0, row[-R]);
 #pragma unroll
-                for (int dx = -R + 1; dx <= R; ++dx) A::badd(t, sg, a, CX0 + dx + R, row[dx]);
+                for (int dx = -R + 1; dx <= R; ++dx) A::sadd(t, a, CX0 + dx + R, row[dx]);
                 A::centre(t, a, IS2D ? 1 : 2, row[0]);
-                xr[i] = A::level(t);
+                xr[i] = A::level(A::send(t));
             }
 #pragma unroll
             for (int v = 0; v < VY; ++v) {
@@ -709,18 +722,16 @@ __device__ __forceinline__ bool stream_item(const Args &a, int bxi, int byi, int
                     q[v][2 * R] = xr[0];
                 } else {
                     float sg = 0.0f;
-                    if constexpr (A::kBounded) {
-                        float b = 0.0f;
+                    if constexpr (A::kAnchored) {
 #pragma unroll
-                        for (int dy = -R; dy <= R; ++dy) b = bound_add(b, coef_abs<C>(a, D + dy + R), xr[v + R + dy]);
-                        sg = sigma_of(b);
+                        for (int dy = -R; dy <= R; ++dy) sg = anchor_add(sg, coef_anchor<C>(a, D + dy + R), xr[v + R + dy]);
                     }
-                    Acc t;
-                    A::bfirst(t, sg, a, D, xr[v]);
+                    typename A::SAcc t;
+                    A::sfirst(t, sg, a, D, xr[v]);
 #pragma unroll
-                    for (int dy = -R + 1; dy <= R; ++dy) A::badd(t, sg, a, D + dy + R, xr[v + R + dy]);
+                    for (int dy = -R + 1; dy <= R; ++dy) A::sadd(t, a, D + dy + R, xr[v + R + dy]);
                     A::centre(t, a, 1, xr[v + R]);
-                    q[v][2 * R] = A::level(t);
+                    q[v][2 * R] = A::level(A::send(t));
                 }
             }
         }
@@ -738,29 +749,29 @@ __device__ __forceinline__ bool stream_item(const Args &a, int bxi, int byi, int
                 // packed: per point the same terms in the same order and the
                 // same roundings.
                 df2 acc[NPR];
+                dfa2 sum[NPR];  // stars and separable passes
                 if constexpr (SEP) {
 #pragma unroll
                     for (int p = 0; p < NPR; ++p) {
                         float b0 = 0.0f, b1 = 0.0f;
 #pragma unroll
                         for (int dz = 0; dz < 2 * R + 1; ++dz) {
-                            const float ch = coef_abs<C>(a, dz);
-                            b0 = bound_add(b0, ch, q[2 * p][dz]);
-                            b1 = bound_add(b1, ch, q[2 * p + 1][dz]);
+                            const float ch = coef_anchor<C>(a, dz);
+                            b0 = anchor_add(b0, ch, q[2 * p][dz]);
+                            b1 = anchor_add(b1, ch, q[2 * p + 1][dz]);
                         }
-                        const u64 sg = pk2(sigma_of(b0), sigma_of(b1));
                         float2 c = coef_f2<C>(a, 0);
-                        dfs2_mul_s(acc[p], sg, c.x, c.y, q[2 * p][0], q[2 * p + 1][0]);
+                        dfa2_first(sum[p], pk2(b0, b1), c.x, c.y, q[2 * p][0], q[2 * p + 1][0]);
 #pragma unroll
                         for (int dz = 1; dz < 2 * R + 1; ++dz) {
                             c = coef_f2<C>(a, dz);
-                            dfs2_fma_s(acc[p], sg, c.x, c.y, q[2 * p][dz], q[2 * p + 1][dz]);
+                            dfa2_add(sum[p], c.x, c.y, q[2 * p][dz], q[2 * p + 1][dz]);
                         }
                     }
                 } else if constexpr (STAR) {
                     const int sl = slot_j >= R ? slot_j - R : slot_j - R + NRING;
                     const TC *pl = cmp_base + sl * CMP_STRIDE;
-                    // each point's sigma from all its inputs
+                    // each point's anchor from all its inputs
                     u64 sg[NPR];
 #pragma unroll
                     for (int p = 0; p < NPR; ++p) {
@@ -768,14 +779,14 @@ __device__ __forceinline__ bool stream_item(const Args &a, int bxi, int byi, int
 #pragma unroll
                         for (int h = 0; h < 2; ++h) {
                             const int v = 2 * p + h;
-                            b[h] = star_bound<C>(a, q[v], pl + own + v * PSTEP);
+                            b[h] = star_anchor<C>(a, q[v], pl + own + v * PSTEP);
                         }
-                        sg[p] = pk2(sigma_of(b[0]), sigma_of(b[1]));
+                        sg[p] = pk2(b[0], b[1]);
                     }
 #pragma unroll
                     for (int p = 0; p < NPR; ++p) {
                         const float2 c = coef_f2<C>(a, coef_slot<C::SHAPE, R>(0, 0, 0));
-                        dfs2_mul_s(acc[p], sg[p], c.x, c.y, q[2 * p][R], q[2 * p + 1][R]);
+                        dfa2_first(sum[p], sg[p], c.x, c.y, q[2 * p][R], q[2 * p + 1][R]);
                     }
 #pragma unroll
                     for (int d = 1; d <= R; ++d)
@@ -783,8 +794,8 @@ __device__ __forceinline__ bool stream_item(const Args &a, int bxi, int byi, int
                         for (int p = 0; p < NPR; ++p) {
                             const float2 cm = coef_f2<C>(a, coef_slot<C::SHAPE, R>(-d, 0, 0));
                             const float2 cp = coef_f2<C>(a, coef_slot<C::SHAPE, R>(d, 0, 0));
-                            dfs2_fma_s(acc[p], sg[p], cm.x, cm.y, q[2 * p][R - d], q[2 * p + 1][R - d]);
-                            dfs2_fma_s(acc[p], sg[p], cp.x, cp.y, q[2 * p][R + d], q[2 * p + 1][R + d]);
+                            dfa2_add(sum[p], cm.x, cm.y, q[2 * p][R - d], q[2 * p + 1][R - d]);
+                            dfa2_add(sum[p], cp.x, cp.y, q[2 * p][R + d], q[2 * p + 1][R + d]);
                         }
                     if constexpr (!IS2D) {
                         TC col[VY + 2 * R];
@@ -796,8 +807,8 @@ __device__ __forceinline__ bool stream_item(const Args &a, int bxi, int byi, int
                             for (int p = 0; p < NPR; ++p) {
                                 const float2 cm = coef_f2<C>(a, coef_slot<C::SHAPE, R>(0, -d, 0));
                                 const float2 cp = coef_f2<C>(a, coef_slot<C::SHAPE, R>(0, d, 0));
-                                dfs2_fma_s(acc[p], sg[p], cm.x, cm.y, col[2 * p + R - d], col[2 * p + 1 + R - d]);
-                                dfs2_fma_s(acc[p], sg[p], cp.x, cp.y, col[2 * p + R + d], col[2 * p + 1 + R + d]);
+                                dfa2_add(sum[p], cm.x, cm.y, col[2 * p + R - d], col[2 * p + 1 + R - d]);
+                                dfa2_add(sum[p], cp.x, cp.y, col[2 * p + R + d], col[2 * p + 1 + R + d]);
                             }
                     }
 #pragma unroll
@@ -807,8 +818,8 @@ __device__ __forceinline__ bool stream_item(const Args &a, int bxi, int byi, int
                             const TC *r0 = pl + own + 2 * p * PSTEP, *r1 = r0 + PSTEP;
                             const float2 cm = coef_f2<C>(a, coef_slot<C::SHAPE, R>(0, 0, -d));
                             const float2 cp = coef_f2<C>(a, coef_slot<C::SHAPE, R>(0, 0, d));
-                            dfs2_fma_s(acc[p], sg[p], cm.x, cm.y, r0[-d], r1[-d]);
-                            dfs2_fma_s(acc[p], sg[p], cp.x, cp.y, r0[d], r1[d]);
+                            dfa2_add(sum[p], cm.x, cm.y, r0[-d], r1[-d]);
+                            dfa2_add(sum[p], cp.x, cp.y, r0[d], r1[d]);
                         }
                 } else {
 #pragma unroll
@@ -837,9 +848,11 @@ __device__ __forceinline__ bool stream_item(const Args &a, int bxi, int byi, int
 #pragma unroll
                 for (int p = 0; p < NPR; ++p) {
                     float h0, h1, l0, l1;
+                    if constexpr (STAR || SEP) acc[p] = dfa2_end(sum[p]);
                     if constexpr (C::ST == kStF32x2) {
                         u64 hh, ll;
-                        renorm2(acc[p], hh, ll);
+                        if constexpr (STAR || SEP) dfa2_renorm(acc[p], hh, ll);
+                        else renorm2(acc[p], hh, ll);
                         upk2(hh, h0, h1);
                         upk2(ll, l0, l1);
                         if (VX == 2 && vmin == 0 && vmax == 2 && (reinterpret_cast<uintptr_t>(optr) & 15u) == 0) {
@@ -865,42 +878,41 @@ __device__ __forceinline__ bool stream_item(const Args &a, int bxi, int byi, int
             }
         } else if (j >= 2 * R) {
             Acc acc[NPT];
+            typename A::SAcc sum[NPT];  // stars and separable passes
             if constexpr (SEP) {
 #pragma unroll
                 for (int v = 0; v < VY; ++v) {
                     float sg = 0.0f;
-                    if constexpr (A::kBounded) {
-                        float b = 0.0f;
+                    if constexpr (A::kAnchored) {
 #pragma unroll
-                        for (int dz = 0; dz < 2 * R + 1; ++dz) b = bound_add(b, coef_abs<C>(a, dz), q[v][dz]);
-                        sg = sigma_of(b);
+                        for (int dz = 0; dz < 2 * R + 1; ++dz) sg = anchor_add(sg, coef_anchor<C>(a, dz), q[v][dz]);
                     }
-                    A::bfirst(acc[v], sg, a, 0, q[v][0]);
+                    A::sfirst(sum[v], sg, a, 0, q[v][0]);
 #pragma unroll
-                    for (int dz = 1; dz < 2 * R + 1; ++dz) A::badd(acc[v], sg, a, dz, q[v][dz]);
-                    A::centre(acc[v], a, 0, q[v][R]);
+                    for (int dz = 1; dz < 2 * R + 1; ++dz) A::sadd(sum[v], a, dz, q[v][dz]);
+                    A::centre(sum[v], a, 0, q[v][R]);
                 }
             } else if constexpr (STAR) {
                 const int sl = slot_j >= R ? slot_j - R : slot_j - R + NRING;
                 const TC *pl = cmp_base + sl * CMP_STRIDE;
-                // each point's sigma from all its inputs (float pairs)
+                // each point's anchor from all its inputs (float pairs)
                 float sg[NPT];
 #pragma unroll
                 for (int v = 0; v < NPT; ++v) {
                     sg[v] = 0.0f;
-                    if constexpr (A::kBounded) sg[v] = sigma_of(star_bound<C>(a, q[v], pl + own + v * PSTEP));
+                    if constexpr (A::kAnchored) sg[v] = star_anchor<C>(a, q[v], pl + own + v * PSTEP);
                 }
 #pragma unroll
                 for (int v = 0; v < NPT; ++v) {
-                    A::bfirst(acc[v], sg[v], a, coef_slot<C::SHAPE, R>(0, 0, 0), q[v][R]);
-                    A::centre(acc[v], a, 0, q[v][R]);
+                    A::sfirst(sum[v], sg[v], a, coef_slot<C::SHAPE, R>(0, 0, 0), q[v][R]);
+                    A::centre(sum[v], a, 0, q[v][R]);
                 }
 #pragma unroll
                 for (int d = 1; d <= R; ++d)
 #pragma unroll
                     for (int v = 0; v < NPT; ++v) {
-                        A::badd(acc[v], sg[v], a, coef_slot<C::SHAPE, R>(-d, 0, 0), q[v][R - d]);
-                        A::badd(acc[v], sg[v], a, coef_slot<C::SHAPE, R>(d, 0, 0), q[v][R + d]);
+                        A::sadd(sum[v], a, coef_slot<C::SHAPE, R>(-d, 0, 0), q[v][R - d]);
+                        A::sadd(sum[v], a, coef_slot<C::SHAPE, R>(d, 0, 0), q[v][R + d]);
                     }
                 if constexpr (!IS2D) {
                     TC col[VY + 2 * R];
@@ -910,8 +922,8 @@ __device__ __forceinline__ bool stream_item(const Args &a, int bxi, int byi, int
                     for (int d = 1; d <= R; ++d)
 #pragma unroll
                         for (int v = 0; v < VY; ++v) {
-                            A::badd(acc[v], sg[v], a, coef_slot<C::SHAPE, R>(0, -d, 0), col[v + R - d]);
-                            A::badd(acc[v], sg[v], a, coef_slot<C::SHAPE, R>(0, d, 0), col[v + R + d]);
+                            A::sadd(sum[v], a, coef_slot<C::SHAPE, R>(0, -d, 0), col[v + R - d]);
+                            A::sadd(sum[v], a, coef_slot<C::SHAPE, R>(0, d, 0), col[v + R + d]);
                         }
                 }
                 if constexpr (IS2D && C::XS) {
@@ -926,8 +938,8 @@ __device__ __forceinline__ bool stream_item(const Args &a, int bxi, int byi, int
                         TC lft = shfl_up_tc(cen, d), rgt = shfl_down_tc(cen, d);
                         if (lane < d) lft = row[-d];
                         if (lane >= 32 - d) rgt = row[d];
-                        A::badd(acc[0], sg[0], a, coef_slot<C::SHAPE, R>(0, 0, -d), lft);
-                        A::badd(acc[0], sg[0], a, coef_slot<C::SHAPE, R>(0, 0, d), rgt);
+                        A::sadd(sum[0], a, coef_slot<C::SHAPE, R>(0, 0, -d), lft);
+                        A::sadd(sum[0], a, coef_slot<C::SHAPE, R>(0, 0, d), rgt);
                     }
                 } else {
 #pragma unroll
@@ -935,8 +947,8 @@ __device__ __forceinline__ bool stream_item(const Args &a, int bxi, int byi, int
 #pragma unroll
                         for (int v = 0; v < NPT; ++v) {
                             const TC *row = pl + own + v * PSTEP;
-                            A::badd(acc[v], sg[v], a, coef_slot<C::SHAPE, R>(0, 0, -d), row[-d]);
-                            A::badd(acc[v], sg[v], a, coef_slot<C::SHAPE, R>(0, 0, d), row[d]);
+                            A::sadd(sum[v], a, coef_slot<C::SHAPE, R>(0, 0, -d), row[-d]);
+                            A::sadd(sum[v], a, coef_slot<C::SHAPE, R>(0, 0, d), row[d]);
                         }
                 }
             } else {
@@ -972,6 +984,10 @@ __device__ __forceinline__ bool stream_item(const Args &a, int bxi, int byi, int
                         }
                     }
                 }
+            }
+            if constexpr (STAR || SEP) {
+#pragma unroll
+                for (int v = 0; v < NPT; ++v) acc[v] = A::send(sum[v]);
             }
             if constexpr (VX == 2 && A::kVecStore) {
                 // two adjacent columns in one vector store when aligned
