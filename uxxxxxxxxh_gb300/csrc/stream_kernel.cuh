@@ -1030,6 +1030,7 @@ __device__ __forceinline__ void stream_cta(const StreamArgs<C::NT> &a) {
         }
         __syncthreads();
     }
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");  // the sweep before has completed
     (void)stream_item<C>(a, blockIdx.x, blockIdx.y, blockIdx.z, smem);
 }
 

@@ -740,6 +740,30 @@ static int stream_occupancy(const StreamCall &c) {
     return occ;
 }
 
+// Estimated time (us) of a streaming launch in z-chunks of zc planes, for
+// choosing shorter chunks on grids too small to fill the GPU.  A CTA walks
+// zc + 2R planes; a plane takes the latency of its load, barrier and sums
+// when the CTA has an SM to itself, and its share of the SM's throughput when
+// K CTAs share one (both matter in between, hence the root of squares).  The
+// rates are GB300's: the FP32 pipe at three quarters (7 operations per term
+// of an anchored sum, 12 of a term-by-term box), FP32 grids at the measured
+// 2.7 to 4.2 points per ns and SM, DFMA at 4 per ns and SM.
+static double stream_estimate(const Plan &pl, const StreamCall &c, int64_t tiles, int64_t nz, int zc, int sms) {
+    int bx, by;
+    stream_tile_xy(c, &bx, &by);
+    const bool is2d = is_rank2_shape(c.shape), df = c.ar == kArDf32, f32 = c.st == kStF32;
+    const bool box = c.shape == kBox3 || c.shape == kBox2, in_place = df && c.st == kStF64;
+    const TileShape t = tile_shape(is2d, box && !is2d && c.R >= 2 ? 3 : c.tile);
+    const double terms = static_cast<double>(pl.coef.size()), w = terms * t.vy * t.vx;
+    const double per_point = f32 ? 0.2 + 0.009 * terms
+                             : df ? (box ? 12.0 * terms : 7.0 * terms + 8.0) / 192.0 + (in_place ? 0.45 : 0.0)
+                                  : terms / 4.0;
+    const double thr = static_cast<double>(bx) * by * per_point * 1e-3;
+    const double lat = f32 ? 0.14 + 0.004 * w : 0.25 + 0.011 * w + (in_place ? 0.15 : 0.0);
+    const double k = static_cast<double>((tiles * ((nz + zc - 1) / zc) + sms - 1) / sms);
+    return (zc + c.R + 1) * std::sqrt(lat * lat + k * thr * k * thr) + 0.1 * k + 1.0;
+}
+
 // z-chunk of a streaming launch: the caller's tile_z, else enough CTAs for
 // about four waves over the SMs, at most the planner's cap; at least 32 rows
 // for rank-2 strips (2048^2 to 4096^2 FP32 5-point: 340 / 507 GStencil/s at
@@ -767,6 +791,22 @@ static int stream_zchunk(const SweepSpec &sp, const Plan &pl, const StreamCall &
             floor_z = std::max(16, 4 * c.R);
         zchunk = static_cast<int>(std::max<int64_t>(floor_z, (nz + chunks - 1) / chunks));
         if (pl.zcap > 0) zchunk = std::min(zchunk, std::max(pl.zcap, floor_z));
+        // Grids below the waves that rule is made for: shorter chunks where
+        // the estimate says at least 3 % (us per sweep at the rule's chunk ->
+        // chosen: 2d1r float pairs 256^2 11.2 -> 2.4, 1024^2 11.3 -> 5.3; 3d1r
+        // 64^3 4.4 -> 2.7, 128^3 8.2 -> 7.3; FP32 256^2 4.7 -> 2.1).
+        if (tiles * ((nz + zchunk - 1) / zchunk) < 4 * slots) {
+            double best = 0.97 * stream_estimate(pl, c, tiles, nz, zchunk, device_sms());
+            const int top = zchunk;
+            for (int z : {2, 3, 4, 6, 8, 12, 16, 24}) {
+                if (z >= top) break;
+                const double est = stream_estimate(pl, c, tiles, nz, z, device_sms());
+                if (est < best) {
+                    best = est;
+                    zchunk = z;
+                }
+            }
+        }
     }
     if (occ_out) *occ_out = occ;
     return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(zchunk > 0 ? zchunk : 1, std::max<int64_t>(nz, 1))));
