@@ -44,8 +44,10 @@ enum : unsigned { kDevErrRange = 1u, kDevErrTimeout = 2u };
 // A status word is kStatusWords unsigned words in device memory:
 //   0 kernel status flags; 1 range-scan largest exponent / halo-check count;
 //   2-7 where the first bounded wait gave up (set, block x, block z, plane,
-//   ring slot, phase); 8 range-scan smallest exponent of a nonzero value.
+//   ring slot, phase); 8 range-scan smallest exponent of a nonzero value;
+//   9-12 a resident run's barrier counters and exponent words (zero between runs).
 constexpr int kStatusWords = 16;
+constexpr int kResidentCtlWord = 9;
 unsigned *stream_error_word(int device, cudaStream_t stream);
 
 // Generic smem plane-ring sweep: any term list, expression order.

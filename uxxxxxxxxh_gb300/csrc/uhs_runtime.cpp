@@ -12,6 +12,7 @@
 //    as it stands (ConvertStencilToStandard.cpp:91-149, 339-381).
 //  * The entry is synchronous for the caller (the MLIR CUDA runtime wrappers
 //    synchronise after each launch); UHS_FLAG_NO_SYNC lifts that.
+#include "resident.h"
 #include "stream_call.h"
 #include "uhs_kernels.h"
 
@@ -82,7 +83,12 @@ unsigned *stream_error_word(int device, cudaStream_t stream) {
     if (it != words.end()) return it->second;
     void *p = nullptr;
     if (dev_alloc(&p, kStatusWords * sizeof(unsigned)) != cudaSuccess) return nullptr;
-    if (cudaMemset(p, 0, kStatusWords * sizeof(unsigned)) != cudaSuccess) {
+    // zeroed on the stream that will use it, in order with its kernels (a
+    // memset captured into a graph would zero it at each replay instead)
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    const bool ordered = cudaStreamIsCapturing(stream, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
+    if ((ordered ? cudaMemsetAsync(p, 0, kStatusWords * sizeof(unsigned), stream)
+                 : cudaMemset(p, 0, kStatusWords * sizeof(unsigned))) != cudaSuccess) {
         cudaFree(p);
         return nullptr;
     }
@@ -691,7 +697,13 @@ static GridView kernel_view(const SweepSpec &sp, const GridView &v) {
 // about 2^169 between its largest (grown) and smallest nonzero magnitudes is
 // the case left to native arithmetic: in float pairs its small cells would
 // keep 24 bits or flush to zero, which a max-normalised error would not show.
-constexpr int kPairLowMargin = 24;
+// log2 of the largest factor T sweeps can grow a magnitude by, (sum |c|)^T
+// where that exceeds 1.
+static double run_growth(const SweepSpec &sp, int T) {
+    double csum = 0.0;
+    for (int k = 0; k < sp.nterms; ++k) csum += std::fabs(sp.coef[k]);
+    return csum > 1.0 ? std::max(T, 1) * std::log2(csum) : 0.0;
+}
 static bool range_ok(const SweepSpec &sp, const GridView &a, const GridView &b, int T, cudaStream_t st,
                      int *shift) {
     *shift = 0;
@@ -710,21 +722,10 @@ static bool range_ok(const SweepSpec &sp, const GridView &a, const GridView &b, 
     if (cudaMemcpyAsync(&e[0], emax, sizeof(unsigned), cudaMemcpyDeviceToHost, st) != cudaSuccess) return false;
     if (cudaMemcpyAsync(&e[1], emin, sizeof(unsigned), cudaMemcpyDeviceToHost, st) != cudaSuccess) return false;
     if (cudaStreamSynchronize(st) != cudaSuccess) return false;
-    if (e[0] >= 0x7ffu) return false;  // Inf or NaN somewhere
-    if (e[1] == 0xffffffffu) return true;  // every cell zero
-    double csum = 0.0;
-    for (int k = 0; k < sp.nterms; ++k) csum += std::fabs(sp.coef[k]);
-    const double growth = csum > 1.0 ? std::max(T, 1) * std::log2(csum) : 0.0;
-    // log2 bound of every magnitude during the run, and the largest scale
-    // that keeps it below 2^120 (kept within +-800 so scaled exponents and
-    // their joins stay inside the FP64 range)
-    const double top = static_cast<double>(static_cast<int>(e[0]) - 1023) + 1.0 + growth;
-    const double sd = std::floor(119.0 - top);
-    if (!(sd >= -800.0)) return false;
-    const int sh = static_cast<int>(std::min(sd, 800.0));
-    if (static_cast<int>(e[1]) - 1023 + sh < -74 + kPairLowMargin) return false;
-    *shift = sh;
-    return true;
+    const PairRange pr = pair_range(static_cast<int>(e[0]), e[1] == 0xffffffffu ? -1 : static_cast<int>(e[1]),
+                                    run_growth(sp, T));
+    *shift = pr.shift;
+    return pr.ok;
 }
 
 // CTAs per SM of a streaming launch's kernel variant (1 when the query fails;
@@ -1013,7 +1014,7 @@ static int launch_fused_pass(const SweepSpec &sp, const Plan &pl, const GridView
 // Read and clear the device error word after the stream drained.
 static int check_status_word(unsigned *w, cudaStream_t st) {
     if (!w) return UHS_OK;
-    unsigned h[8] = {};
+    unsigned h[kStatusWords] = {};
     cudaError_t e = cudaMemcpyAsync(h, w, sizeof h, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return cuda_error(e, "device status read");
@@ -1643,6 +1644,84 @@ static cudaError_t dev_alloc_async(void **p, size_t bytes, cudaStream_t st) {
     return e;
 }
 
+// A run held in shared memory from its first sweep to its last (resident.cuh):
+// rank-2 star and box programs of two or more sweeps on FP64 (UHS_ARITH_AUTO) and
+// FP32 grids whose domain fits, when the caller and the tuner database leave
+// the launch to the backend.  *ran stays false when it does not apply, or
+// its scratch or its launch could not be had, and the sweeps are launched one
+// by one; with *native set, the data's range needs native FP64 arithmetic
+// (both grids are then as they were).
+static int run_resident(const SweepSpec &sp, const Plan &pl, const uhs_params *p, const GridView &va,
+                        const GridView &vb, int T, cudaStream_t st, bool *ran, bool *native) {
+    *ran = false;
+    *native = false;
+    const bool f64 = pl.st == kStF64;
+    const int other = UHS_FLAG_IN_PLACE | UHS_FLAG_XSHUFFLE;
+    // FP64 from two sweeps on (the range scan and the conversions go too: 256^2
+    // to 1448^2, T = 4, 70-110 us a run against 95-150); FP32 from eight: at T
+    // = 4 its set-up costs what the launches do (48-83 against 45-75 us).
+    if (T < (f64 ? 2 : 8) || sp.rank != 2 || pl.kernel != UHS_KERNEL_STREAM || !params_are_auto(p) || (p && (p->flags & other)) ||
+        (f64 ? !pl.auto_df32 : pl.st != kStF32))
+        return UHS_OK;
+    const int64_t nz = sp.ub[1] - sp.lb[1], nx = sp.ub[2] - sp.lb[2];
+    const int cell = f64 ? 8 : 4;
+    const ResPlan rp = plan_resident(pl.shape != kStar2, pl.R, cell, static_cast<int>(pl.coef.size()), nz, nx,
+                                     device_sms(), kResidentSmem);
+    if (rp.px == 0) return UHS_OK;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) {
+        cudaGetLastError();
+        return UHS_OK;
+    }
+    if (cap != cudaStreamCaptureStatusNone) return UHS_OK;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    unsigned *err = stream_error_word(dev, st);
+    if (!err) return UHS_OK;  // the sweeps report it
+    const size_t bytes = static_cast<size_t>(nz * nx) * 4 * cell;  // {value, step} words, two buffers
+    void *buf = nullptr;
+    if (dev_alloc_async(&buf, bytes + 256, st) != cudaSuccess) return UHS_OK;
+    const GridView ka = kernel_view(sp, va), kb = kernel_view(sp, vb);
+    ResCall c{};
+    c.a = ka.data;
+    c.b = kb.data;
+    c.as0 = ka.s[0];
+    c.bs0 = kb.s[0];
+    c.lb0 = static_cast<int>(sp.lb[1]);
+    c.lb2 = static_cast<int>(sp.lb[2]);
+    c.nz = static_cast<int>(nz);
+    c.nx = static_cast<int>(nx);
+    c.pz = rp.pz;
+    c.px = rp.px;
+    c.G = rp.G;
+    c.L = rp.L;
+    c.halo_off = rp.halo_off;
+    c.T = T;
+    c.round64 = f64 && T < kPairMinT ? 1 : 0;
+    c.growth = run_growth(sp, T);
+    c.pub = buf;
+    c.ctl = err + kResidentCtlWord;
+    c.err = err;
+    c.verdict = reinterpret_cast<int *>(static_cast<char *>(buf) + bytes);
+    const cudaError_t e = launch_resident(pl.shape, pl.R, pl.st, c, rp.smem, pl.coef.data(), st);
+    if (e != cudaSuccess) {
+        cudaGetLastError();  // not sticky: the caller launches the sweeps
+        cudaFreeAsync(buf, st);
+        return UHS_OK;
+    }
+    *ran = true;
+    int rc = UHS_OK;
+    if (f64) {
+        int verdict = 0;
+        cudaError_t ce = cudaMemcpyAsync(&verdict, c.verdict, sizeof verdict, cudaMemcpyDeviceToHost, st);
+        if (ce == cudaSuccess) ce = cudaStreamSynchronize(st);
+        if (ce != cudaSuccess) rc = cuda_error(ce, "resident run");
+        else *native = verdict == 2;
+    }
+    cudaFreeAsync(buf, st);
+    return rc;
+}
+
 // Pair-resident run of a float-pair FP64 program (see uhs_run in uhs.h):
 // *ran stays false when the scratch could not be had or planned, and the
 // caller then sweeps the FP64 grids in place.
@@ -1913,7 +1992,12 @@ int uhs_run(const uhs_stencil_desc *d, const uhs_memref *a, const uhs_memref *b,
     Plan pl;
     if ((rc = plan_sweep(sp, p, va, &pl))) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (pl.auto_df32 && d->iterations > 0 && !range_ok(sp, va, vb, d->iterations, st, &pl.pair_shift)) {
+    bool resident = false, native = false;
+    rc = run_resident(sp, pl, p, va, vb, d->iterations, st, &resident, &native);
+    if (rc) return rc;
+    if (resident && !native) return finish(p, st);
+    if (pl.auto_df32 && d->iterations > 0 &&
+        (native || !range_ok(sp, va, vb, d->iterations, st, &pl.pair_shift))) {
         fall_back_native(pl);
     }
     if (pl.kernel == UHS_KERNEL_STREAM && pl.cfg.k_temporal > 1 && d->iterations > 1) {
