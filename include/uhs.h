@@ -56,9 +56,10 @@ enum {
 
 enum {
     UHS_ARITH_AUTO = 0,  /* the backend picks: for F64 grids on the streaming kernel,
-                            float pairs scaled by a power of two chosen from a device
-                            scan of both grids (one extra read of each grid and one
-                            host round trip per call), unless the grids hold Inf/NaN
+                            float pairs scaled by a power of two chosen by a device
+                            scan of the cells the program reads (one extra read of a;
+                            the call waits for its verdict, also with
+                            UHS_FLAG_NO_SYNC), unless they hold Inf/NaN
                             or span more than about 2^169 between the largest
                             magnitude grown by (sum|c|)^T and the smallest nonzero
                             one; then UHS_ARITH_FMA */
@@ -197,19 +198,27 @@ int uhs_validate(const uhs_stencil_desc *desc, const uhs_memref *a, const uhs_me
  * the program reads.
  *
  * Pair-resident runs: FP64 grids swept in float-pair arithmetic (UHS_ARITH_AUTO
- * after its range check, or UHS_ARITH_DF32) with T >= 8 sweeps on the
- * streaming kernel (star and box stencils) run on float-pair copies of the grids.  Each value is split into its {hi, lo}
- * floats once, the T sweeps read and write pairs, and the domain of both grids
- * is joined back to FP64 at the end.  The halo is read from the FP64 grids and
- * never written, so it stays bit-exact.  The copies (16 bytes per grid cell)
+ * or UHS_ARITH_DF32) with T >= 8 sweeps on the streaming kernel (star and box
+ * stencils; under UHS_ARITH_AUTO also T >= 4 on 2^21 points or more) run on
+ * float-pair copies of the grids.  Under UHS_ARITH_AUTO the first sweep splits
+ * each value of a into its {hi, lo} floats as it reads them and the last two
+ * join theirs as they write b and a; only the cells around the domain are
+ * copied beforehand.  (UHS_ARITH_DF32, and term-by-term 3D boxes of radius 2-3,
+ * split and join in passes of their own.)  The halo is read from the FP64
+ * grids and never written, so it stays bit-exact.  The copies (16 bytes per
+ * cell, rows padded to whole 128-byte lines)
  * are stream-ordered allocations from a memory pool the library owns on each
  * device, which keeps freed memory for the next run (uhs_release_scratch
  * returns it; the device's default pool is not touched).  When that
  * allocation fails, or with UHS_FLAG_IN_PLACE, the sweeps run on the FP64
- * grids directly, splitting on every load.
+ * grids directly, splitting on every load.  FP32 programs whose rows the
+ * hardware cannot load in whole lines run on padded FP32 copies (8 bytes per
+ * cell) in the same way, when the launch is left to the backend and the run is
+ * long enough to pay for them.
  *
  * Range: under UHS_ARITH_AUTO the pairs hold every value times 2^s, with s
- * chosen from a scan of both grids so that the largest magnitude, grown by
+ * chosen from a scan of the cells the program reads (a's domain and both
+ * grids' cells around it) so that the largest magnitude, grown by
  * (sum|c|)^T, stays below 2^120 (a linear sweep commutes with the scale
  * exactly); the run keeps float pairs when every nonzero magnitude, scaled,
  * is at least 2^-50, and computes in native FP64 otherwise (or when a grid

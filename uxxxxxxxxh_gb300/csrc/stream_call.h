@@ -16,6 +16,13 @@ constexpr bool is_rank2_shape(int shape) { return shape == kStar2 || shape == kB
 enum { kStF64 = 0, kStF32 = 1, kStF32x2 = 2 };
 enum { kArNative = 0, kArDf32 = 1 };
 enum { kLdCpAsync = 0, kLdTma = 1 };
+enum { kIoPlain = 0, kIoFirst = 1, kIoLast = 2 };
+// The range scan's verdict on an FP64 run (range_scan.cu), read by its kernels.
+enum { kRunPairs = 1, kRunNative = 2 };
+struct PairRun {
+    int state;
+    int bias;  // exponent rebias of the run's pairs (pair_bias, df32.cuh)
+};
 // Term capacity of a batched grid's arguments (the 7x7x7 box).
 constexpr int kBatchNT = 343;
 
@@ -38,6 +45,9 @@ struct StreamArgs {
     // element of the output row (vector stores); cells left of lb2 are not
     // written
     int xoff;
+    const PairRun *run;  // FP64 runs in float pairs decided on the device (NULL: pair_shift holds)
+    float2 *out2;        // kIoLast: the pairs too (NULL: FP64 only)
+    int64_t out2_s0, out2_s1;
     unsigned *err;
     double cd[NT];
     float2 chl[NT];  // float rounding of each coefficient and its rounding error (hi, lo)
@@ -83,6 +93,9 @@ struct StreamCall {
     int pair_shift;  // FP64 grids in float pairs: power-of-two scale of the pairs (0: none)
     int xshuffle;    // rank-2 stars: x-neighbours by warp shuffles (UHS_FLAG_XSHUFFLE)
     int xoff;        // two points per thread along x: tile origin lb[2] - xoff (StreamArgs::xoff)
+    int io;          // kIo*
+    const PairRun *run;
+    GridView out2;   // kIoLast: the pairs' grid (data NULL: none)
     unsigned *err;
     cudaStream_t stream;
     int *occ_out;  // when set: report CTAs per SM of the variant instead of launching
@@ -124,6 +137,10 @@ cudaError_t launch_stream_f64n_2d(const StreamCall &c);
 cudaError_t launch_stream_f64df_2d(const StreamCall &c);
 cudaError_t launch_stream_f32_2d(const StreamCall &c);
 cudaError_t launch_stream_f32x2_2d(const StreamCall &c);
+// First and last sweeps of runs on float-pair copies (kIoFirst, kIoLast): the
+// planner's default tiles, kIoLast by TMA (term-by-term 2D boxes: cp.async).
+cudaError_t launch_stream_ends_3d(const StreamCall &c);
+cudaError_t launch_stream_ends_2d(const StreamCall &c);
 
 // Geometry of a variant as the kernel template computes it (host mirror).
 inline void stream_box(const StreamCall &c, int eb, int *W, int *H) {

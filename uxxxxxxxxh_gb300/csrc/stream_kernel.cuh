@@ -76,15 +76,25 @@ __host__ __device__ constexpr int coef_slot(int dz, int dy, int dx) {
 // XS: rank-2 stars take their x-neighbours by warp shuffles (UHS_FLAG_XSHUFFLE).
 // VX: points per thread along x (rank-2 stars: 1 or 2); a CTA tile is
 // CX = BX * VX columns wide.
+// IO: what the sweep reads and writes.  kIoPlain: grids of one type.  The ends
+// of a run on float-pair copies: kIoFirst reads the FP64 grid and writes
+// pairs, kIoLast reads pairs and writes the FP64 grid (and, for step T - 1,
+// the pairs too, StreamArgs::out2).
 template <int SHAPE_, int R_, int ST_, int AR_, int LD_, int BX_, int TYT_, int VY_, int PD_, int XS_ = 0,
-          int VX_ = 1>
+          int VX_ = 1, int IO_ = kIoPlain>
 struct StreamCfg {
     static constexpr int SHAPE = SHAPE_, R = R_, ST = ST_, AR = AR_, LD = LD_, BX = BX_, TYT = TYT_, VY = VY_,
-                         PD = PD_, XS = XS_, VX = VX_;
+                         PD = PD_, XS = XS_, VX = VX_, IO = IO_;
+    static_assert(IO == kIoPlain || AR == kArDf32, "run ends: float pairs");
     static constexpr int CX = BX * VX;
     using SI = ShapeInfo<SHAPE, R>;
     using TS = std::conditional_t<ST == kStF64, double, std::conditional_t<ST == kStF32, float, float2>>;
     static constexpr bool CONVERT = (ST == kStF64 && AR == kArDf32);
+    // element type written
+    using TO = std::conditional_t<IO == kIoFirst, float2, std::conditional_t<IO == kIoLast, double, TS>>;
+    static constexpr bool OUT_PAIRS = std::is_same_v<TO, float2>;
+    // float pairs joined to FP64 on store
+    static constexpr bool JOIN = AR == kArDf32 && std::is_same_v<TO, double>;
     using TC = std::conditional_t<CONVERT, float2, TS>;
     static constexpr int EB = sizeof(TS);
     static constexpr int Q = 16 / EB;  // TMA x-coordinate granule, elements
@@ -342,8 +352,8 @@ struct Arith<C, kArDf32> {
     // x * 2^pair_shift).  A sum that outgrew the float range (hi Inf or NaN)
     // would join to a finite double; it sets the range flag instead of
     // passing unnoticed.
-    __device__ static __forceinline__ void store(typename C::TS *p, const Acc &acc, unsigned &range_err, int bias) {
-        if constexpr (C::ST == kStF64) {
+    __device__ static __forceinline__ void store(typename C::TO *p, const Acc &acc, unsigned &range_err, int bias) {
+        if constexpr (C::JOIN) {
             range_err |= (__float_as_uint(acc.h) & 0x7f800000u) == 0x7f800000u;
             *p = join_f64(acc.h, acc.l, bias);
         } else {
@@ -351,9 +361,9 @@ struct Arith<C, kArDf32> {
         }
     }
     static constexpr bool kVecStore = true;
-    __device__ static __forceinline__ void store2(typename C::TS *p, const Acc &a0, const Acc &a1, unsigned &range_err,
+    __device__ static __forceinline__ void store2(typename C::TO *p, const Acc &a0, const Acc &a1, unsigned &range_err,
                                                   int bias) {
-        if constexpr (C::ST == kStF64) {
+        if constexpr (C::JOIN) {
             range_err |= (__float_as_uint(a0.h) & 0x7f800000u) == 0x7f800000u;
             range_err |= (__float_as_uint(a1.h) & 0x7f800000u) == 0x7f800000u;
             *reinterpret_cast<double2 *>(p) = make_double2(join_f64(a0.h, a0.l, bias), join_f64(a1.h, a1.l, bias));
@@ -400,6 +410,14 @@ __device__ __forceinline__ float star_anchor(const Args &a, const TC *zq, const 
     return b;
 }
 
+// Exponent rebias of the run's pairs: the device's verdict on the grids' range
+// (PairRun) or the host's.
+template <class Args>
+__device__ __forceinline__ int run_bias(const Args &a) {
+    if constexpr (std::is_same_v<Args, BatchArgs>) return pair_bias(a.pair_shift);
+    else return a.run ? a.run->bias : pair_bias(a.pair_shift);
+}
+
 // ---- the kernel ---------------------------------------------------------
 // One work item: the (bx, by) tile of the (y, x) plane over z-chunk bz.
 // Returns false when a bounded wait ran out (the status word is set).
@@ -409,6 +427,7 @@ template <class C, class Args>
 __device__ __forceinline__ bool stream_item(const Args &a, int bxi, int byi, int bzi, unsigned char *smem) {
     using TS = typename C::TS;
     using TC = typename C::TC;
+    using TO = typename C::TO;
     using A = Arith<C>;
     using Acc = typename A::Acc;
     constexpr int R = C::R, RY = C::RY, BX = C::BX, TYT = C::TYT, VY = C::VY, W = C::W, H = C::H;
@@ -569,7 +588,16 @@ __device__ __forceinline__ bool stream_item(const Args &a, int bxi, int byi, int
     // output pointer of (zs, y0 + ty*VY, x0 + VX*tx); points vmin..vmax-1
     // are written: rows beyond ub1 are masked, and with two points along x
     // columns beyond ub2 and the column left of lb2 (xoff)
-    TS *optr = static_cast<TS *>(a.out) + zs * a.out_s0 + (y0 + ty * VY) * a.out_s1 + x0 + VX * tx;
+    TO *optr = static_cast<TO *>(a.out) + zs * a.out_s0 + (y0 + ty * VY) * a.out_s1 + x0 + VX * tx;
+    // step T - 1 of a run on copies: the pairs as well
+    [[maybe_unused]] float2 *optr2 = nullptr;
+    [[maybe_unused]] int64_t ostep2 = 1;
+    if constexpr (C::IO == kIoLast) {
+        if (a.out2) optr2 = a.out2 + zs * a.out2_s0 + (y0 + ty * VY) * a.out2_s1 + x0 + VX * tx;
+        ostep2 = VX == 2 ? 1 : a.out2_s1;
+    }
+    [[maybe_unused]] int bias = 0;
+    if constexpr (C::CONVERT || C::JOIN) bias = run_bias(a);
     int vmax = VX == 2 ? static_cast<int>(min(static_cast<int64_t>(2), a.ub2 - (x0 + 2 * tx)))
                        : static_cast<int>(min(static_cast<int64_t>(VY), a.ub1 - (y0 + ty * VY)));
     if (!x_ok) vmax = 0;
@@ -628,7 +656,7 @@ __device__ __forceinline__ bool stream_item(const Args &a, int bxi, int byi, int
 #pragma unroll
                     for (int c0 = 0; c0 < WL; c0 += BX)
                         if (c0 + tx < WL)
-                            dp[r * W + c0 + tx] = split_f64(sp[r * W + c0 + tx], range_err, pair_bias(a.pair_shift));
+                            dp[r * W + c0 + tx] = split_f64(sp[r * W + c0 + tx], range_err, bias);
                 }
             }
             __syncthreads();
@@ -849,7 +877,18 @@ __device__ __forceinline__ bool stream_item(const Args &a, int bxi, int byi, int
                 for (int p = 0; p < NPR; ++p) {
                     float h0, h1, l0, l1;
                     if constexpr (STAR || SEP) acc[p] = dfa2_end(sum[p]);
-                    if constexpr (C::ST == kStF32x2) {
+                    if constexpr (C::IO == kIoLast) {
+                        if (optr2) {
+                            u64 hh, ll;
+                            if constexpr (STAR || SEP) dfa2_renorm(acc[p], hh, ll);
+                            else renorm2(acc[p], hh, ll);
+                            upk2(hh, h0, h1);
+                            upk2(ll, l0, l1);
+                            if (2 * p >= vmin && 2 * p < vmax) optr2[2 * p * ostep2] = make_float2(h0, l0);
+                            if (2 * p + 1 < vmax) optr2[(2 * p + 1) * ostep2] = make_float2(h1, l1);
+                        }
+                    }
+                    if constexpr (C::OUT_PAIRS) {
                         u64 hh, ll;
                         if constexpr (STAR || SEP) dfa2_renorm(acc[p], hh, ll);
                         else renorm2(acc[p], hh, ll);
@@ -865,16 +904,19 @@ __device__ __forceinline__ bool stream_item(const Args &a, int bxi, int byi, int
                         upk2(acc[p].h, h0, h1);
                         upk2(acc[p].l, l0, l1);
                         if (VX == 2 && vmin == 0 && vmax == 2 && (reinterpret_cast<uintptr_t>(optr) & 15u) == 0) {
-                            A::store2(optr, df{h0, l0}, df{h1, l1}, range_err, pair_bias(a.pair_shift));
+                            A::store2(optr, df{h0, l0}, df{h1, l1}, range_err, bias);
                         } else {
                             if (2 * p >= vmin && 2 * p < vmax)
-                                A::store(optr + 2 * p * ostep, df{h0, l0}, range_err, pair_bias(a.pair_shift));
+                                A::store(optr + 2 * p * ostep, df{h0, l0}, range_err, bias);
                             if (2 * p + 1 < vmax)
-                                A::store(optr + (2 * p + 1) * ostep, df{h1, l1}, range_err, pair_bias(a.pair_shift));
+                                A::store(optr + (2 * p + 1) * ostep, df{h1, l1}, range_err, bias);
                         }
                     }
                 }
                 optr += a.out_s0;
+                if constexpr (C::IO == kIoLast) {
+                    if (optr2) optr2 += a.out2_s0;
+                }
             }
         } else if (j >= 2 * R) {
             Acc acc[NPT];
@@ -989,18 +1031,26 @@ __device__ __forceinline__ bool stream_item(const Args &a, int bxi, int byi, int
 #pragma unroll
                 for (int v = 0; v < NPT; ++v) acc[v] = A::send(sum[v]);
             }
+            if constexpr (C::IO == kIoLast) {
+                if (optr2) {
+#pragma unroll
+                    for (int v = 0; v < NPT; ++v)
+                        if (v >= vmin && v < vmax) optr2[v * ostep2] = A::level(acc[v]);
+                    optr2 += a.out2_s0;
+                }
+            }
             if constexpr (VX == 2 && A::kVecStore) {
                 // two adjacent columns in one vector store when aligned
-                if (vmin == 0 && vmax == 2 && (reinterpret_cast<uintptr_t>(optr) & (2 * sizeof(TS) - 1)) == 0)
-                    A::store2(optr, acc[0], acc[1], range_err, pair_bias(a.pair_shift));
+                if (vmin == 0 && vmax == 2 && (reinterpret_cast<uintptr_t>(optr) & (2 * sizeof(TO) - 1)) == 0)
+                    A::store2(optr, acc[0], acc[1], range_err, bias);
                 else
 #pragma unroll
                     for (int v = 0; v < NPT; ++v)
-                        if (v >= vmin && v < vmax) A::store(optr + v * ostep, acc[v], range_err, pair_bias(a.pair_shift));
+                        if (v >= vmin && v < vmax) A::store(optr + v * ostep, acc[v], range_err, bias);
             } else {
 #pragma unroll
                 for (int v = 0; v < NPT; ++v)
-                    if (v >= vmin && v < vmax) A::store(optr + v * ostep, acc[v], range_err, pair_bias(a.pair_shift));
+                    if (v >= vmin && v < vmax) A::store(optr + v * ostep, acc[v], range_err, bias);
             }
             optr += a.out_s0;
         }
@@ -1010,7 +1060,7 @@ __device__ __forceinline__ bool stream_item(const Args &a, int bxi, int byi, int
         s_iss = s_iss + 1 == NSTG ? 0 : s_iss + 1;
         if constexpr (C::CONVERT) s_cmp = s_cmp + 1 == NCMP ? 0 : s_cmp + 1;
     }
-    if constexpr (C::CONVERT) {
+    if constexpr (C::CONVERT || C::JOIN) {
         if (range_err) atomicOr(a.err, kDevErrRange);
     }
     __syncthreads();
@@ -1031,6 +1081,10 @@ __device__ __forceinline__ void stream_cta(const StreamArgs<C::NT> &a) {
         __syncthreads();
     }
     asm volatile("griddepcontrol.wait;\n" ::: "memory");  // the sweep before has completed
+    // the range scan found that the run needs native FP64: leave both grids as they are
+    if constexpr (C::AR == kArDf32) {
+        if (a.run && a.run->state != kRunPairs) return;
+    }
     (void)stream_item<C>(a, blockIdx.x, blockIdx.y, blockIdx.z, smem);
 }
 

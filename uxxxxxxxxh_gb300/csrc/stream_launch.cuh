@@ -34,6 +34,12 @@ cudaError_t launch_cfg(const StreamCall &c) {
     a.pair_loads = c.pair_loads;
     a.pair_shift = c.pair_shift;
     a.xoff = C::VX == 2 ? c.xoff : 0;
+    a.run = c.run;
+    if (C::IO == kIoLast) {
+        a.out2 = static_cast<float2 *>(c.out2.data);
+        a.out2_s0 = c.out2.s[0];
+        a.out2_s1 = c.out2.s[1];
+    }
     a.err = c.err;
     fill_coefs(a.cd, a.chl, a.cl_sum, c.coef, C::NT, c.shape, c.R);
     fill_coef_anchor(a.cab, a.chl, C::NT);

@@ -45,9 +45,10 @@ enum : unsigned { kDevErrRange = 1u, kDevErrTimeout = 2u };
 //   0 kernel status flags; 1 range-scan largest exponent / halo-check count;
 //   2-7 where the first bounded wait gave up (set, block x, block z, plane,
 //   ring slot, phase); 8 range-scan smallest exponent of a nonzero value;
-//   9-12 a resident run's barrier counters and exponent words (zero between runs).
+//   9-12 the barrier counters and exponent words of resident runs and run scans
+//   (zero between launches).
 constexpr int kStatusWords = 16;
-constexpr int kResidentCtlWord = 9;
+constexpr int kRunCtlWord = 9;
 unsigned *stream_error_word(int device, cudaStream_t stream);
 
 // Generic smem plane-ring sweep: any term list, expression order.
@@ -108,6 +109,19 @@ cudaError_t launch_from_pairs(const GridView &src, const GridView &dst, const in
 // exponent 0) into *min_out (atomicMin; must start at 0xffffffff).
 cudaError_t launch_exponent_range(const void *data, int64_t n_words, unsigned *max_out, unsigned *min_out, int sms,
                                   cudaStream_t st);
+
+// Range scan of an FP64 run on the device (range_scan.cu): a's domain and the
+// shells (within `reach` of the domain) of a and b (NULL: a alone) decide
+// float pairs or native, and the pairs' scale, into *run for the run's
+// kernels.  ctl: four words of the stream, zero between launches.
+struct PairRun;
+cudaError_t launch_run_scan(const GridView &a, const GridView *b, const int64_t lb[3], const int64_t ub[3],
+                            const int reach[3], double growth, unsigned *ctl, PairRun *run, cudaStream_t st);
+// Shells of both grids into a run's own copies (domain origin clb in those):
+// FP64 split into pairs by *run, or FP32 cells.
+cudaError_t launch_shell_copy(bool f64, const GridView &a, const GridView &b, const GridView &ca, const GridView &cb,
+                              const int64_t lb[3], const int64_t ub[3], const int64_t clb[3], const int reach[3],
+                              const PairRun *run, cudaStream_t st);
 
 // FP32 3D box stencils of radius 2 and 3 on the tensor cores (box_mma.cu).
 // Coefficients in box slot order ((dz+R)*D + (dy+R))*D + (dx+R), D = 2R+1.

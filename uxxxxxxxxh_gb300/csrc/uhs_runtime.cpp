@@ -219,6 +219,7 @@ struct Plan {
     bool factored = false;     // separable box run as 1D passes
     bool a_tmem = false;       // tensor-core path: A operand staged in tensor memory
     bool xshuffle = false;     // rank-2 stars: x-neighbours by warp shuffles
+    const PairRun *run = nullptr;  // FP64 in float pairs decided on the device (launch_run_scan)
 };
 
 int device_sm_count() {
@@ -664,6 +665,7 @@ static bool make_tmap(const GridView &v, int eb, int W, int H, CUtensorMap *m) {
 
 static cudaError_t stream_dispatch(const StreamCall &c) {
     const bool is2d = is_rank2_shape(c.shape);
+    if (c.io != kIoPlain) return is2d ? launch_stream_ends_2d(c) : launch_stream_ends_3d(c);
     if (c.st == kStF64 && c.ar == kArNative) return is2d ? launch_stream_f64n_2d(c) : launch_stream_f64n_3d(c);
     if (c.st == kStF64) return is2d ? launch_stream_f64df_2d(c) : launch_stream_f64df_3d(c);
     if (c.st == kStF32) return is2d ? launch_stream_f32_2d(c) : launch_stream_f32_3d(c);
@@ -834,6 +836,69 @@ static StreamCall stream_call_of(const SweepSpec &sp, const Plan &pl) {
     return c;
 }
 
+// FP32 rows loaded by cp.async: 8-byte pairs when every row of every tile
+// starts 8-byte aligned.
+static bool rows_load_in_pairs(const StreamCall &c, int64_t tile_x0) {
+    return (tile_x0 - c.R) % 2 == 0 && c.in.s[0] % 2 == 0 && c.in.s[1] % 2 == 0 && c.in.n[2] % 2 == 0 &&
+           reinterpret_cast<uintptr_t>(c.in.data) % 8 == 0;
+}
+
+// A streaming sweep ready to launch, once or on every step of a run.
+struct StreamLaunch {
+    StreamCall c{};
+    CUtensorMap tmap;
+    StreamLaunch() = default;
+    StreamLaunch(const StreamLaunch &) = delete;
+    StreamLaunch &operator=(const StreamLaunch &) = delete;
+    int launch() const {
+        const cudaError_t e = stream_dispatch(c);
+        return e == cudaSuccess ? UHS_OK : cuda_error(e, "streaming sweep launch");
+    }
+};
+
+// in and out are indexed with the same coordinates, sp's domain.
+static int prepare_stream(const SweepSpec &sp, const Plan &pl, const GridView &in, const GridView &out,
+                          cudaStream_t st, unsigned *err_word, int io, StreamLaunch *l) {
+    StreamCall &c = l->c;
+    c = stream_call_of(sp, pl);
+    c.io = io;
+    c.in = kernel_view(sp, in);
+    c.out = kernel_view(sp, out);
+    const bool is2d = sp.rank == 2;
+    c.stream = st;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    c.err = err_word ? err_word : stream_error_word(dev, st);
+    c.pair_shift = pl.pair_shift;
+    c.run = pl.run;
+    if (!c.err) return set_error(UHS_ENOMEM, "device error word allocation failed");
+    const int eb = sp.dtype == UHS_F32 ? 4 : 8;
+    // two points per thread along x: start the tiles on an even element of
+    // the output's first row (vector stores of each thread's pair)
+    c.xoff = 0;
+    if (is2d && tile_shape(true, c.tile).vx == 2) {
+        const int64_t e0 = static_cast<int64_t>(reinterpret_cast<uintptr_t>(c.out.data) / eb) + c.lb[0] * c.out.s[0] +
+                           c.lb[2];
+        c.xoff = static_cast<int>(e0 & 1);
+    }
+    const int64_t tile_x0 = c.lb[2] - c.xoff;  // first column of the first tile
+    if (c.ld == kLdTma) {
+        int W, H;
+        stream_box(c, eb, &W, &H);
+        if (make_tmap(c.in, eb, W, H, &l->tmap)) {
+            c.tmap = &l->tmap;
+            const int q = 16 / eb;
+            c.shift = static_cast<int>(((tile_x0 - c.R) % q + q) % q);
+        } else {
+            c.ld = kLdCpAsync;
+        }
+    }
+    c.zchunk = stream_zchunk(sp, pl, c, nullptr);
+    // 4-byte grids: copy in 8-byte pairs when every row start of the tile is 8-byte aligned
+    if (eb == 4 && c.ld == kLdCpAsync) c.pair_loads = rows_load_in_pairs(c, tile_x0) ? 1 : 0;
+    return UHS_OK;
+}
+
 static int launch_sweep(const SweepSpec &sp, const Plan &pl, const GridView &in, const GridView &out,
                         cudaStream_t st, unsigned *err_word = nullptr) {
     if (pl.kernel == UHS_KERNEL_GENERIC) {
@@ -862,62 +927,9 @@ static int launch_sweep(const SweepSpec &sp, const Plan &pl, const GridView &in,
         if (e != cudaSuccess) return cuda_error(e, "tensor-core box sweep launch");
         return UHS_OK;
     }
-    StreamCall c{};
-    c.shape = pl.shape;
-    c.R = pl.R;
-    c.st = pl.st;
-    c.ar = pl.ar;
-    c.ld = pl.ld;
-    c.tile = pl.tile;
-    c.coef = pl.coef.data();
-    c.in = kernel_view(sp, in);
-    c.out = kernel_view(sp, out);
-    const bool is2d = sp.rank == 2;
-    c.lb[0] = is2d ? sp.lb[1] : sp.lb[0];
-    c.ub[0] = is2d ? sp.ub[1] : sp.ub[0];
-    c.lb[1] = is2d ? 0 : sp.lb[1];
-    c.ub[1] = is2d ? 1 : sp.ub[1];
-    c.lb[2] = sp.lb[2];
-    c.ub[2] = sp.ub[2];
-    c.stream = st;
-    int dev = 0;
-    cudaGetDevice(&dev);
-    c.err = err_word ? err_word : stream_error_word(dev, st);
-    c.pair_shift = pl.pair_shift;
-    c.xshuffle = pl.xshuffle ? 1 : 0;
-    if (!c.err) return set_error(UHS_ENOMEM, "device error word allocation failed");
-    const int eb = sp.dtype == UHS_F32 ? 4 : 8;
-    // two points per thread along x: start the tiles on an even element of
-    // the output's first row (vector stores of each thread's pair)
-    c.xoff = 0;
-    if (is2d && tile_shape(true, c.tile).vx == 2) {
-        const int64_t e0 = static_cast<int64_t>(reinterpret_cast<uintptr_t>(c.out.data) / eb) + c.lb[0] * c.out.s[0] +
-                           c.lb[2];
-        c.xoff = static_cast<int>(e0 & 1);
-    }
-    const int64_t tile_x0 = c.lb[2] - c.xoff;  // first column of the first tile
-    CUtensorMap tmap;
-    if (c.ld == kLdTma) {
-        int W, H;
-        stream_box(c, eb, &W, &H);
-        if (make_tmap(c.in, eb, W, H, &tmap)) {
-            c.tmap = &tmap;
-            const int q = 16 / eb;
-            c.shift = static_cast<int>(((tile_x0 - c.R) % q + q) % q);
-        } else {
-            c.ld = kLdCpAsync;
-        }
-    }
-    c.zchunk = stream_zchunk(sp, pl, c, nullptr);
-    // 4-byte grids: copy in 8-byte pairs when every row start of the tile is 8-byte aligned
-    if (eb == 4 && c.ld == kLdCpAsync) {
-        const bool even = ((tile_x0 - c.R) % 2 == 0) && c.in.s[0] % 2 == 0 && c.in.s[1] % 2 == 0 &&
-                          c.in.n[2] % 2 == 0 && reinterpret_cast<uintptr_t>(c.in.data) % 8 == 0;
-        c.pair_loads = even ? 1 : 0;
-    }
-    cudaError_t e = stream_dispatch(c);
-    if (e != cudaSuccess) return cuda_error(e, "streaming sweep launch");
-    return UHS_OK;
+    StreamLaunch l;
+    const int rc = prepare_stream(sp, pl, in, out, st, err_word, kIoPlain, &l);
+    return rc ? rc : l.launch();
 }
 
 // Pass depths for T steps with fusion depth k (1, 2 or 4).  Passes alternate
@@ -1644,6 +1656,16 @@ static cudaError_t dev_alloc_async(void **p, size_t bytes, cudaStream_t st) {
     return e;
 }
 
+// The device's verdict on an FP64 run's range, once its stream has drained.
+static int read_verdict(const int *state, cudaStream_t st, bool *native) {
+    int v = 0;
+    cudaError_t e = cudaMemcpyAsync(&v, state, sizeof v, cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) return cuda_error(e, "range verdict");
+    *native = v == kRunNative;
+    return UHS_OK;
+}
+
 // A run held in shared memory from its first sweep to its last (resident.cuh):
 // rank-2 star and box programs of two or more sweeps on FP64 (UHS_ARITH_AUTO) and
 // FP32 grids whose domain fits, when the caller and the tuner database leave
@@ -1700,7 +1722,7 @@ static int run_resident(const SweepSpec &sp, const Plan &pl, const uhs_params *p
     c.round64 = f64 && T < kPairMinT ? 1 : 0;
     c.growth = run_growth(sp, T);
     c.pub = buf;
-    c.ctl = err + kResidentCtlWord;
+    c.ctl = err + kRunCtlWord;
     c.err = err;
     c.verdict = reinterpret_cast<int *>(static_cast<char *>(buf) + bytes);
     const cudaError_t e = launch_resident(pl.shape, pl.R, pl.st, c, rp.smem, pl.coef.data(), st);
@@ -1710,16 +1732,199 @@ static int run_resident(const SweepSpec &sp, const Plan &pl, const uhs_params *p
         return UHS_OK;
     }
     *ran = true;
-    int rc = UHS_OK;
+    const int rc = f64 ? read_verdict(c.verdict, st, native) : UHS_OK;
+    cudaFreeAsync(buf, st);
+    return rc;
+}
+
+// Elements from one grid's cell to another's of the same domain coordinates:
+// out as seen by a kernel that indexes it with in's coordinates.
+static GridView shifted_view(const GridView &g, const int64_t from[3], const int64_t to[3], int eb) {
+    GridView v = g;
+    v.data = static_cast<char *>(g.data) +
+             ((to[0] - from[0]) * g.s[0] + (to[1] - from[1]) * g.s[1] + (to[2] - from[2])) * eb;
+    return v;
+}
+
+// Runs of FP64 grids in float pairs on the library's own copies (pairs,
+// UHS_ARITH_AUTO) and FP32 runs on padded copies (star, separable and small
+// term-by-term box programs on the streaming kernel).
+//
+// The copies hold the domain and the cells within R of it, rows padded so
+// that TMA loads them whatever the caller's pitch and every row of the domain
+// starts on a 128-byte line.  The first sweep reads the caller's grid and the
+// last ones write it, so no pass converts or copies a domain; only the shells
+// are copied.  FP64: the range scan decides on the device (PairRun) and the
+// host learns of it at the end, no round trip in between.
+//
+// us per sweep, float pairs / FP32 grids, caller's layout -> copies: 3d2r star
+// 97 x 131 x 203 24.2 / 14.5 (207-cell rows: 8- and 4-byte cp.async) -> 14.7 /
+// 7.7; 3d1r star 200 x 200 x 201 38.3 / 24.5 -> 27 / 13; 3d1r star 512^3 364 /
+// 210 -> 337 / 176 (aligned lines).
+//
+// FP64 runs of T >= kPairMinT take copies as before; shorter ones (T >= 4) from
+// kSoloPoints points on, where the grid is out of L2 and an in-place sweep
+// costs a third more than a pair sweep (8192^2 T = 4, 3d1r 512^3 T = 4); below
+// that size they keep the in-place sweeps, whose results round to FP64 between
+// steps like the batched kernel's.  FP32 pays an extra sweep (step T - 1 goes
+// to the copy and to b) and the shell copy.  3D rows that TMA cannot load: us a
+// run, sweeps alone -> copies, 3d2r star T = 20: 64^2 x 65 145 -> 120, 100^2 x
+// 101 210 -> 165, 160^2 x 161 430 -> 271; T = 8: 81 -> 83, 113 -> 102; so from
+// 2^18 points at T >= 16, 2^20 at T >= 8.  Rows that TMA loads, or that 8-byte
+// cp.async pairs do for radius 1-2, only miss the lines: radius 1 out of L2
+// (512^3 T = 50 10.5 -> 9.3 ms; 3d1r at 129^2 x 130 T = 20 147 -> 163 us, 64^3
+// 87 -> 95).  2D rows that cannot load in 8-byte pairs: 3000 x 3001 21.9 -> 19.3
+// us a sweep.
+static int run_on_copies(const SweepSpec &sp, const Plan &pl, const uhs_params *p, const GridView &va,
+                         const GridView &vb, int T, cudaStream_t st, bool *ran, bool *native) {
+    *ran = false;
+    *native = false;
+    const bool f64 = pl.st == kStF64, is2d = sp.rank == 2;
+    const int R = pl.R;
+    if (T < 4 || pl.kernel != UHS_KERNEL_STREAM || pl.cfg.k_temporal > 1 || pl.cfg.use_tma < 0 ||
+        (p && (p->flags & UHS_FLAG_IN_PLACE)) || (pl.shape == kBox3 && R >= 2))
+        return UHS_OK;
+    int64_t n[3], points = 1;
+    for (int i = 0; i < 3; ++i) points *= n[i] = sp.ub[i] - sp.lb[i];
+    if (points <= 0) return UHS_OK;
     if (f64) {
-        int verdict = 0;
-        cudaError_t ce = cudaMemcpyAsync(&verdict, c.verdict, sizeof verdict, cudaMemcpyDeviceToHost, st);
-        if (ce == cudaSuccess) ce = cudaStreamSynchronize(st);
-        if (ce != cudaSuccess) rc = cuda_error(ce, "resident run");
-        else *native = verdict == 2;
+        if (!pl.auto_df32 || (T < kPairMinT && points < kSoloPoints)) return UHS_OK;
+    } else {
+        if (pl.st != kStF32 || !params_are_auto(p) || (p && (p->flags & UHS_FLAG_XSHUFFLE))) return UHS_OK;
+        StreamCall c = stream_call_of(sp, pl);
+        c.in = kernel_view(sp, va);
+        const bool tma = pl.ld == kLdTma, in_pairs = rows_load_in_pairs(c, c.lb[2]);
+        if (is2d ? T < 16 || tma || in_pairs
+            : tma || (in_pairs && R <= 2) ? R > 1 || T < 16 || points < (int64_t(1) << 24)
+                                          : T < 8 || points < (int64_t(1) << (T < 16 ? 20 : 18)))
+            return UHS_OK;
+    }
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) {
+        cudaGetLastError();
+        return UHS_OK;
+    }
+    if (cap != cudaStreamCaptureStatusNone) return UHS_OK;
+    // the copies: domain origin clb, 128-byte lines (2D FP32 strips: an even
+    // distance from the first column loaded)
+    const int cell = f64 ? 8 : 4, line = 128 / cell;
+    const int reach[3] = {is2d ? 0 : R, R, R};
+    const int64_t lead = !f64 && is2d ? line + R % 2 : line;
+    const int64_t clb[3] = {reach[0], R, lead};
+    const int64_t m0 = n[0] + 2 * reach[0], m1 = n[1] + 2 * R, m2 = (lead + n[2] + R + line - 1) / line * line;
+    if (m1 * m2 >= (int64_t(1) << 31)) return UHS_OK;
+    SweepSpec sp2 = sp;
+    if (f64) sp2.dtype = UHS_F32X2;
+    for (int i = 0; i < 3; ++i) {
+        sp2.lb[i] = clb[i];
+        sp2.ub[i] = clb[i] + n[i];
+    }
+    int dev = 0;
+    cudaGetDevice(&dev);
+    unsigned *err = stream_error_word(dev, st);
+    if (!err) return UHS_OK;  // the sweeps report it
+    const size_t bytes = static_cast<size_t>(m0 * m1 * m2) * cell;
+    void *buf = nullptr;
+    if (dev_alloc_async(&buf, 2 * bytes + 256, st) != cudaSuccess) return UHS_OK;
+    const GridView pa{buf, {m0, m1, m2}, {m1 * m2, m2, 1}};
+    const GridView pb{static_cast<char *>(buf) + bytes, {m0, m1, m2}, {m1 * m2, m2, 1}};
+    PairRun *const run = f64 ? reinterpret_cast<PairRun *>(static_cast<char *>(buf) + 2 * bytes) : nullptr;
+    // plans: the sweeps between with the caller's parameters, the first and
+    // last ones with the defaults they are built for
+    uhs_params q, ends;
+    if (p) q = *p;
+    else uhs_params_default(&q);
+    uhs_params_default(&ends);
+    ends.flags = q.flags & UHS_FLAG_NO_FACTOR;
+    if (f64) q.arith = ends.arith = UHS_ARITH_DF32;
+    Plan mid, first, last;
+    StreamLaunch l_first, l_ab, l_ba, l_b, l_a;
+    bool ready;
+    {
+        ErrorMessageGuard keep;
+        ready = plan_sweep(sp2, &q, pa, &mid) == UHS_OK && mid.kernel == UHS_KERNEL_STREAM &&
+                plan_sweep(sp, &ends, va, &first) == UHS_OK && first.kernel == UHS_KERNEL_STREAM &&
+                plan_sweep(sp2, &ends, pa, &last) == UHS_OK && last.kernel == UHS_KERNEL_STREAM;
+        mid.run = first.run = last.run = run;
+        const GridView wb = shifted_view(vb, clb, sp.lb, cell), wa = shifted_view(va, clb, sp.lb, cell);
+        ready = ready &&
+                prepare_stream(sp, first, va, shifted_view(pb, sp.lb, clb, cell), st, err, f64 ? kIoFirst : kIoPlain,
+                               &l_first) == UHS_OK &&
+                prepare_stream(sp2, mid, pa, pb, st, err, kIoPlain, &l_ab) == UHS_OK &&
+                prepare_stream(sp2, mid, pb, pa, st, err, kIoPlain, &l_ba) == UHS_OK &&
+                prepare_stream(sp2, last, pa, wb, st, err, f64 ? kIoLast : kIoPlain, &l_b) == UHS_OK &&
+                prepare_stream(sp2, last, pb, wa, st, err, f64 ? kIoLast : kIoPlain, &l_a) == UHS_OK;
+        // the float-pair end sweeps load by TMA (2D boxes term by term: cp.async)
+        if (f64 && pl.shape != kBox2) ready = ready && l_b.c.ld == kLdTma && l_a.c.ld == kLdTma;
+    }
+    if (!ready) {
+        cudaFreeAsync(buf, st);
+        return UHS_OK;
+    }
+    *ran = true;
+    int rc = UHS_OK;
+    cudaError_t e = cudaSuccess;
+    if (f64) {
+        l_b.c.out2 = kernel_view(sp2, pb);
+        e = launch_run_scan(va, &vb, sp.lb, sp.ub, reach, run_growth(sp, T), err + kRunCtlWord, run, st);
+    }
+    if (e == cudaSuccess) e = launch_shell_copy(f64, va, vb, pa, pb, sp.lb, sp.ub, clb, reach, run, st);
+    if (e != cudaSuccess) rc = cuda_error(e, "run set-up");
+    if (!rc) rc = l_first.launch();
+    for (int t = 2; t <= T - 2 && !rc; ++t) rc = (t % 2 ? l_ab : l_ba).launch();
+    // step T - 1 into b, and into the copy that step T reads
+    if (!rc && !f64) rc = l_ab.launch();
+    if (!rc) rc = l_b.launch();
+    if (!rc) rc = l_a.launch();
+    if (f64) {
+        const int vrc = read_verdict(&run->state, st, native);
+        if (!rc) rc = vrc;
     }
     cudaFreeAsync(buf, st);
     return rc;
+}
+
+// FP64 sweeps in place under UHS_ARITH_AUTO (T = 0: one sweep a -> b, as T = 1;
+// b's shell is not read then): the range scan decides on the device, the
+// sweeps follow it, and the host learns of it at the end.  *ran stays false
+// when the word for the verdict cannot be had.
+static int run_in_place_scanned(const SweepSpec &sp, const Plan &pl, const GridView &va, const GridView &vb, int T,
+                                cudaStream_t st, bool *ran, bool *native) {
+    *ran = false;
+    *native = false;
+    if (!pl.auto_df32 || pl.kernel != UHS_KERNEL_STREAM || pl.cfg.k_temporal > 1) return UHS_OK;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) {
+        cudaGetLastError();
+        return UHS_OK;
+    }
+    if (cap != cudaStreamCaptureStatusNone) return UHS_OK;
+    for (int i = 0; i < 3; ++i)
+        if (sp.ub[i] <= sp.lb[i]) return UHS_OK;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    unsigned *err = stream_error_word(dev, st);
+    void *buf = nullptr;
+    if (!err || dev_alloc_async(&buf, 256, st) != cudaSuccess) return UHS_OK;
+    Plan scanned = pl;
+    PairRun *const run = static_cast<PairRun *>(buf);
+    scanned.run = run;
+    const int reach[3] = {sp.rank == 2 ? 0 : pl.R, pl.R, pl.R};
+    StreamLaunch ab, ba;
+    int rc = prepare_stream(sp, scanned, va, vb, st, err, kIoPlain, &ab);
+    if (!rc && T > 1) rc = prepare_stream(sp, scanned, vb, va, st, err, kIoPlain, &ba);
+    if (rc) {
+        cudaFreeAsync(buf, st);
+        return rc;
+    }
+    *ran = true;
+    const cudaError_t e =
+        launch_run_scan(va, T > 1 ? &vb : nullptr, sp.lb, sp.ub, reach, run_growth(sp, T), err + kRunCtlWord, run, st);
+    if (e != cudaSuccess) rc = cuda_error(e, "range scan");
+    for (int t = 0; t < std::max(T, 1) && !rc; ++t) rc = (t % 2 ? ba : ab).launch();
+    const int vrc = read_verdict(&run->state, st, native);
+    cudaFreeAsync(buf, st);
+    return rc ? rc : vrc;
 }
 
 // Pair-resident run of a float-pair FP64 program (see uhs_run in uhs.h):
@@ -1762,10 +1967,10 @@ static int run_pair_resident(const SweepSpec &sp, const uhs_params *p, const Gri
     cudaError_t e = launch_to_pairs(va, pa, sp.lb, sp.ub, false, shift, err, st);
     if (e == cudaSuccess) e = launch_to_pairs(vb, pb, sp.lb, sp.ub, true, shift, err, st);
     if (e != cudaSuccess) rc = cuda_error(e, "float-pair conversion");
-    for (int it = 0; it < T / 2 && rc == UHS_OK; ++it) {
-        if ((rc = launch_sweep(sp2, pl2, pa, pb, st))) break;
-        rc = launch_sweep(sp2, pl2, pb, pa, st);
-    }
+    StreamLaunch ab, ba;
+    if (rc == UHS_OK) rc = prepare_stream(sp2, pl2, pa, pb, st, err, kIoPlain, &ab);
+    if (rc == UHS_OK) rc = prepare_stream(sp2, pl2, pb, pa, st, err, kIoPlain, &ba);
+    for (int t = 0; t < T && rc == UHS_OK; ++t) rc = (t % 2 ? ba : ab).launch();
     if (rc == UHS_OK) {
         e = launch_from_pairs(pa, va, sp.lb, sp.ub, shift, err, st);
         if (e == cudaSuccess) e = launch_from_pairs(pb, vb, sp.lb, sp.ub, shift, err, st);
@@ -1973,7 +2178,10 @@ int uhs_sweep(const uhs_stencil_desc *d, const uhs_memref *in, const uhs_memref 
     Plan pl;
     if ((rc = plan_sweep(sp, p, vi, &pl))) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (pl.auto_df32 && !range_ok(sp, vi, vo, 1, st, &pl.pair_shift)) {
+    bool done = false, native = false;
+    if ((rc = run_in_place_scanned(sp, pl, vi, vo, 1, st, &done, &native))) return rc;
+    if (done && !native) return finish(p, st);
+    if (pl.auto_df32 && (native || !range_ok(sp, vi, vo, 1, st, &pl.pair_shift))) {
         fall_back_native(pl);
     }
     if ((rc = launch_sweep(sp, pl, vi, vo, st))) return rc;
@@ -1992,10 +2200,15 @@ int uhs_run(const uhs_stencil_desc *d, const uhs_memref *a, const uhs_memref *b,
     Plan pl;
     if ((rc = plan_sweep(sp, p, va, &pl))) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    bool resident = false, native = false;
-    rc = run_resident(sp, pl, p, va, vb, d->iterations, st, &resident, &native);
-    if (rc) return rc;
-    if (resident && !native) return finish(p, st);
+    // on chip, on the library's copies, or in place under the device's range
+    // verdict; a run whose range needs native FP64 has left the grids as they were
+    bool done = false, native = false;
+    if ((rc = run_resident(sp, pl, p, va, vb, d->iterations, st, &done, &native))) return rc;
+    if (!done && (rc = run_on_copies(sp, pl, p, va, vb, d->iterations, st, &done, &native))) return rc;
+    if (!done && d->iterations > 0 && !pair_eligible(pl, d->iterations, p) &&
+        (rc = run_in_place_scanned(sp, pl, va, vb, d->iterations, st, &done, &native)))
+        return rc;
+    if (done && !native) return finish(p, st);
     if (pl.auto_df32 && d->iterations > 0 &&
         (native || !range_ok(sp, va, vb, d->iterations, st, &pl.pair_shift))) {
         fall_back_native(pl);
@@ -2023,6 +2236,12 @@ int uhs_run(const uhs_stencil_desc *d, const uhs_memref *a, const uhs_memref *b,
     }
     if (d->iterations == 1) {
         if ((rc = launch_sweep(sp, pl, va, vb, st))) return rc;
+    } else if (pl.kernel == UHS_KERNEL_STREAM) {
+        StreamLaunch ab, ba;
+        if ((rc = prepare_stream(sp, pl, va, vb, st, nullptr, kIoPlain, &ab))) return rc;
+        if ((rc = prepare_stream(sp, pl, vb, va, st, nullptr, kIoPlain, &ba))) return rc;
+        for (int t = 0; t < d->iterations; ++t)
+            if ((rc = (t % 2 ? ba : ab).launch())) return rc;
     } else {
         for (int it = 0; it < d->iterations / 2; ++it) {
             if ((rc = launch_sweep(sp, pl, va, vb, st))) return rc;
