@@ -306,4 +306,21 @@ __device__ __forceinline__ void dfa2_renorm(const df2 &a, u64 &h, u64 &l) {
     l = sub2(a.l, sub2(h, a.h));
 }
 
+// acc += g, an (unnormalised) pair: TwoSum of the high parts.  Adds a group of
+// terms summed on its own anchor to a longer sum.
+__device__ __forceinline__ void df_add(df &acc, df g) {
+    const float s = __fadd_rn(acc.h, g.h);
+    const float v = __fsub_rn(s, acc.h);
+    const float t = __fadd_rn(__fsub_rn(acc.h, __fsub_rn(s, v)), __fsub_rn(g.h, v));
+    acc.h = s;
+    acc.l = __fadd_rn(acc.l, __fadd_rn(t, g.l));
+}
+__device__ __forceinline__ void df2_add(df2 &acc, const df2 &g) {
+    const u64 s = add2(acc.h, g.h);
+    const u64 v = sub2(s, acc.h);
+    const u64 t = add2(sub2(acc.h, sub2(s, v)), sub2(g.h, v));
+    acc.h = s;
+    acc.l = add2(acc.l, add2(t, g.l));
+}
+
 }  // namespace uhs

@@ -124,11 +124,20 @@ struct StreamCfg {
     // sums in both: stars on float-pair grids r1/r2/r3 330/184/129
     // -> 341/186/134 (best tiles), on FP64 grids 169/114/86 -> 191/130/97;
     // separable boxes FP64 141/92/63 -> 163/102/68; radius-3 boxes 5.5/6.0 ->
-    // 7.5/7.2.  Term-by-term boxes of radius 1 on float-pair grids (100 ->
-    // 96) and of radius 2 (21.2 -> 20.4, FP64 19.3 -> 19.0) keep the scalar
-    // sums.
+    // 7.5/7.2.  Term-by-term boxes of radius 1-2 on float-pair grids keep the
+    // scalar sums (r1 100 -> 96; r2, grouped sums, 26.5 -> 26.4; FP64 grids in
+    // place r2 23.8 -> 25.7).
     static constexpr bool PACKED = AR == kArDf32 && (SI::is2d ? VX == 2 : VY % 2 == 0) &&
-                                   !(SHAPE == kBox3 && (R == 2 || (R == 1 && ST == kStF32x2)));
+                                   !(SHAPE == kBox3 && R <= 2 && ST == kStF32x2);
+    // Term-by-term 3D boxes of radius 2-3 in float pairs: each column of 2R + 1
+    // terms is an anchored sum of its own, and the columns are joined by TwoSum
+    // (8.7 / 8.2 FP32 operations per term instead of 12; GStencil/s at 256^3 r2 /
+    // r3 21.9 / 7.7 -> 26.5 / 9.7).  More accurate than
+    // TwoSum per term there (rms error / B of random sums, in 2^-49: 125 terms
+    // 13.3 -> 3.8 for one sign, 2.3 -> 1.6 mixed; 343 terms 36 -> 6.1, 3.7 ->
+    // 1.8); not for 2D boxes or 27 terms of mixed signs (25 terms 1.3 -> 2.3,
+    // 27 terms 1.34 -> 1.54), which keep it.
+    static constexpr bool GROUPED = AR == kArDf32 && SHAPE == kBox3 && R >= 2;
     static_assert(LD != kLdTma || W <= 256, "TMA boxes are at most 256 elements wide");
     static_assert(!SI::is2d || (TYT == 1 && VY == 1), "rank-2 tiles are one row");
     static_assert(!XS || (SI::is2d && SI::star), "lane shuffles: rank-2 stars");
@@ -860,6 +869,29 @@ __device__ __forceinline__ bool stream_item(const Args &a, int bxi, int byi, int
                             TC col[VY + 2 * R];
 #pragma unroll
                             for (int i = 0; i < VY + 2 * R; ++i) col[i] = pl[own + (i - R) * W + dx];
+                            if constexpr (C::GROUPED) {
+#pragma unroll
+                                for (int p = 0; p < NPR; ++p) {
+                                    float b0 = 0.0f, b1 = 0.0f;
+#pragma unroll
+                                    for (int dy = -R; dy <= R; ++dy) {
+                                        const float ch = coef_anchor<C>(a, coef_slot<C::SHAPE, R>(dz, dy, dx));
+                                        b0 = anchor_add(b0, ch, col[2 * p + R + dy]);
+                                        b1 = anchor_add(b1, ch, col[2 * p + 1 + R + dy]);
+                                    }
+                                    dfa2 g;
+                                    float2 c = coef_f2<C>(a, coef_slot<C::SHAPE, R>(dz, -R, dx));
+                                    dfa2_first(g, pk2(b0, b1), c.x, c.y, col[2 * p], col[2 * p + 1]);
+#pragma unroll
+                                    for (int dy = -R + 1; dy <= R; ++dy) {
+                                        c = coef_f2<C>(a, coef_slot<C::SHAPE, R>(dz, dy, dx));
+                                        dfa2_add(g, c.x, c.y, col[2 * p + R + dy], col[2 * p + 1 + R + dy]);
+                                    }
+                                    if (dz == -R && dx == -R) acc[p] = dfa2_end(g);
+                                    else df2_add(acc[p], dfa2_end(g));
+                                }
+                                continue;
+                            }
 #pragma unroll
                             for (int dy = -R; dy <= R; ++dy)
 #pragma unroll
@@ -1013,6 +1045,24 @@ __device__ __forceinline__ bool stream_item(const Args &a, int bxi, int byi, int
                             TC col[VY + 2 * R];
 #pragma unroll
                             for (int i = 0; i < VY + 2 * R; ++i) col[i] = pl[own + (i - R) * W + dx];
+                            if constexpr (C::GROUPED) {
+#pragma unroll
+                                for (int v = 0; v < VY; ++v) {
+                                    float sg = 0.0f;
+#pragma unroll
+                                    for (int dy = -R; dy <= R; ++dy)
+                                        sg = anchor_add(sg, coef_anchor<C>(a, coef_slot<C::SHAPE, R>(dz, dy, dx)),
+                                                        col[v + R + dy]);
+                                    typename A::SAcc g;
+                                    A::sfirst(g, sg, a, coef_slot<C::SHAPE, R>(dz, -R, dx), col[v]);
+#pragma unroll
+                                    for (int dy = -R + 1; dy <= R; ++dy)
+                                        A::sadd(g, a, coef_slot<C::SHAPE, R>(dz, dy, dx), col[v + R + dy]);
+                                    if (dz == -R && dx == -R) acc[v] = A::send(g);
+                                    else df_add(acc[v], A::send(g));
+                                }
+                                continue;
+                            }
 #pragma unroll
                             for (int dy = -R; dy <= R; ++dy)
 #pragma unroll
