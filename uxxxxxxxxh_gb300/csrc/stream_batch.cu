@@ -90,6 +90,7 @@ __global__ void __launch_bounds__(256, 3) k_stream_batch(const BatchGrid *__rest
     __shared__ int skind;
     __shared__ int snext;
     const int tid = threadIdx.y * blockDim.x + threadIdx.x;
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");  // the timestep before has completed
     for (;;) {
         if (tid == 0) snext = atomicAdd(counter, 1);
         __syncthreads();
@@ -141,9 +142,9 @@ int batch_kind(int pack, int shape, int R, int st, int ar) {
     return -1;
 }
 
-// 32-plane z-chunks: longer chunks re-read fewer halo planes but give fewer,
-// longer items; on GB300 16, 24, 32 and 16(R+1) planes timed within 2 % on
-// the 64-grid suite, and 32 was fastest.
+// The longest z-chunks (the runtime shortens them to the batch's work): 32
+// planes re-read few halo planes; on GB300 16, 24, 32 and 16(R+1) planes timed
+// within 2 % on the 64-grid suite, and 32 was fastest.
 void batch_tile(int shape, int R, int st, int *bx, int *by, int *zchunk) {
     if (is_rank2_shape(shape)) {
         *bx = 256;
@@ -164,12 +165,22 @@ cudaError_t batch_prepare(int pack, BatchPackInfo *info) {
 cudaError_t batch_launch(int pack, const BatchGrid *grids, const int4 *items, int n_items, int dir, int ctas,
                          int *counter, cudaStream_t st) {
     if (n_items <= 0) return cudaSuccess;
-    if (pack == kPackMain)
-        k_stream_batch<MainPack><<<ctas, dim3(32, 8), MainPack::SMEM, st>>>(grids, items, n_items, dir, counter);
-    else
-        k_stream_batch<NativePack><<<ctas, dim3(32, 8), NativePack::SMEM, st>>>(grids, items, n_items, dir, counter);
-    count_launch();
-    return cudaGetLastError();
+    // programmatic dependent launch, as the standalone sweeps (stream_launch.cuh)
+    cudaLaunchConfig_t lc{};
+    lc.gridDim = dim3(static_cast<unsigned>(ctas));
+    lc.blockDim = dim3(32, 8);
+    lc.dynamicSmemBytes = pack == kPackMain ? MainPack::SMEM : NativePack::SMEM;
+    lc.stream = st;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    lc.attrs = &at;
+    lc.numAttrs = 1;
+    const cudaError_t e =
+        cudaLaunchKernelEx(&lc, pack == kPackMain ? k_stream_batch<MainPack> : k_stream_batch<NativePack>, grids,
+                           items, n_items, dir, counter);
+    if (e == cudaSuccess) count_launch();
+    return e;
 }
 
 void batch_fill_args(BatchArgs *a, const StreamCall &c, int nt) {

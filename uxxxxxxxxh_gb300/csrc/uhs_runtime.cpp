@@ -1123,17 +1123,24 @@ struct BatchGridHost {
     int pack, kind, T, order;
     int bx, by, zc;    // item tile and z-chunk
     int64_t items;
-    double item_cost;  // estimated cost of one item, for the list order
+    int R;
+    double plane_us;   // estimated time of a plane, and of an item (list order)
+    double item_cost;
 };
 
-// Relative cost of one work item: points per item x (per-point overhead +
-// terms x per-term cost of the arithmetic).  Per-term costs follow the
-// measured rates of the streaming kernels (FP32 FFMA 1, float pairs about
-// 6 FP32 operations' worth, native FP64 bound by the FP64 pipe).
-static double batch_item_cost(int bx, int by, int zc, int nterms, int st, int ar) {
-    const double per_term = st == kStF32 ? 1.0 : ar == kArDf32 ? 6.0 : 14.0;
-    return static_cast<double>(bx) * by * zc * (20.0 + per_term * nterms);
+// Time (us) of one plane (row, rank 2) of a work item on an SM of its own:
+// its loads, barrier and sums, fitted to GB300 batches of one grid (2D 256^2,
+// 3D 40^3; e.g. FP64 3d1r / 3d3r star 1.3 / 4.3, 3d2r / 3d3r box 4.0 / 9.6,
+// FP32 0.7 / 1.0, 2.7 / 6.3).  Items share SMs, so this orders and balances
+// them rather than predicts.
+static double batch_plane_us(int shape, int st, int ar, int nterms) {
+    const bool is2d = is_rank2_shape(shape), box = shape == kBox3 || shape == kBox2;
+    if (st == kStF32) return is2d ? 0.25 + 0.01 * nterms : 0.5 + 0.017 * nterms;
+    if (ar == kArNative) return is2d ? 0.3 + 0.035 * nterms : 0.3 + 0.07 * nterms;
+    return is2d ? 0.4 + 0.025 * nterms : box ? 3.0 + 0.02 * nterms : 0.2 * nterms;
 }
+// An item walks zc planes and the R before and after them, and starts up.
+static double batch_item_us(double plane_us, int R, int zc) { return plane_us * (zc + 0.5 * R + 1.5); }
 
 // Grids of at least kSoloPoints interior points run in a batch as their own
 // sweep launches -- the standalone plan: tuner-database or default tile,
@@ -1284,7 +1291,7 @@ static int batch_create(const uhs_stencil_desc *descs, const uhs_memref *as, con
                 }
             }
             solo.push_back(g);
-            info[i] = BatchGridHost{-1, 0, 0, i, 1, 1, 1, 0, 0.0};
+            info[i] = BatchGridHost{-1, 0, 0, i, 1, 1, 1, 0, 0, 0.0, 0.0};
             continue;
         }
         uhs_params bp;
@@ -1333,29 +1340,54 @@ static int batch_create(const uhs_stencil_desc *descs, const uhs_memref *as, con
             batch_fill_args(&host[i].dir[d], c, static_cast<int>(pl.coef.size()));
         }
         host[i].kind = kind;
-        info[i] = BatchGridHost{pack, kind, descs[i].iterations, i, bx, by, zc, 0,
-                                batch_item_cost(bx, by, 1, static_cast<int>(pl.coef.size()), pl.st, pl.ar)};
+        info[i] = BatchGridHost{pack, kind, descs[i].iterations, i, bx, by, zc, 0, pl.R,
+                                batch_plane_us(pl.shape, pl.st, pl.ar, static_cast<int>(pl.coef.size())), 0.0};
     }
-    // z-chunks: the batch's estimated work shared by every resident CTA sets
-    // a target item cost; grids whose 32-plane items would exceed a quarter of
-    // a CTA's share get shorter chunks (down to 8 planes), so no single long
-    // item holds up the end of a timestep.
+    // z-chunks: a timestep ends with its longest item or with the last slot's
+    // share of all of them.  For a few bounds on an item's time, every grid
+    // takes its longest chunk within the bound (down to one plane); the bound
+    // with the shortest estimated timestep holds.  ms per 20 steps against
+    // items of at least 8 planes: 24 grids of sides 64-512 / 16-64 6.7 -> 1.34,
+    // 64 of them 7.5 -> 2.4, 32 grids of 500-1400 / 90-125 15.2 -> 13.2.  (An
+    // 8-plane item of a 343-term FP64 box takes 110 us by itself.)
     {
-        double work = 0.0;
-        for (int i = 0; i < n; ++i) {
-            if (info[i].pack < 0) continue;  // solo grid
+        const double slots = 3.0 * device_sms();
+        const auto tiles = [&](int i) {
             const BatchArgs &a0 = host[i].dir[0];
-            work += info[i].item_cost * static_cast<double>((a0.ub2 - a0.lb2) * (a0.ub1 - a0.lb1)) /
-                    (static_cast<double>(info[i].bx) * info[i].by) * static_cast<double>(a0.ub0 - a0.lb0);
+            return static_cast<double>(((a0.ub2 - a0.lb2 + info[i].bx - 1) / info[i].bx) *
+                                       ((a0.ub1 - a0.lb1 + info[i].by - 1) / info[i].by));
+        };
+        const auto chunk = [&](const BatchGridHost &g, double bound) {
+            int zc = g.zc;
+            while (zc > 1 && batch_item_us(g.plane_us, g.R, zc) > bound) zc = zc > 8 ? zc / 2 : zc - 1;
+            return zc;
+        };
+        double best = 1e300, best_bound = 1e300;
+        for (double bound = 2.0; bound < 600.0; bound *= 1.41) {
+            double longest = 0.0, total = 0.0;
+            for (int i = 0; i < n; ++i) {
+                if (info[i].pack < 0) continue;  // solo grid
+                const BatchArgs &a0 = host[i].dir[0];
+                const int64_t nz = a0.ub0 - a0.lb0;
+                const int zc = chunk(info[i], bound);
+                const double us = batch_item_us(info[i].plane_us, info[i].R, static_cast<int>(std::min<int64_t>(zc, nz)));
+                longest = std::max(longest, us);
+                total += us * tiles(i) * static_cast<double>((nz + zc - 1) / zc);
+            }
+            // the slots' share, and the last item past it (weights of the share
+            // from 0.7 to 3 on 18 batches: 0.7 and 1 within 1 %, 2 and 3 6-9 % slower)
+            const double est = total / slots + longest;
+            if (est < best) {
+                best = est;
+                best_bound = bound;
+            }
         }
-        const double target = work / (4.0 * device_sms() * 3);
         for (int i = 0; i < n; ++i) {
             BatchGridHost &g = info[i];
             if (g.pack < 0) continue;
-            int zc = g.zc;
-            while (zc > 8 && g.item_cost * zc > target) zc /= 2;
+            const int zc = chunk(g, best_bound);
             g.zc = zc;
-            g.item_cost *= zc;
+            g.item_cost = batch_item_us(g.plane_us, g.R, zc);
             for (int d = 0; d < 2; ++d) host[i].dir[d].zchunk = zc;
             const BatchArgs &a0 = host[i].dir[0];
             const int64_t tx = (a0.ub2 - a0.lb2 + g.bx - 1) / g.bx, ty = (a0.ub1 - a0.lb1 + g.by - 1) / g.by,
