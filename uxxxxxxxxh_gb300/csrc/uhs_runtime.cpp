@@ -1023,15 +1023,51 @@ static int launch_fused_pass(const SweepSpec &sp, const Plan &pl, const GridView
     return UHS_OK;
 }
 
-// Read and clear the device error word after the stream drained.
-static int check_status_word(unsigned *w, cudaStream_t st) {
-    if (!w) return UHS_OK;
-    unsigned h[kStatusWords] = {};
-    cudaError_t e = cudaMemcpyAsync(h, w, sizeof h, cudaMemcpyDeviceToHost, st);
+// Pinned words each host thread reads a stream's results into: the copies of
+// a call's end are enqueued together and waited for once (pageable copies are
+// staged and waited for one by one, 5-10 us each).  Freed with the thread.
+constexpr int kEndWords = kStatusWords + 1;
+static unsigned *pinned_end_words() {
+    struct Words {
+        unsigned *p = nullptr;
+        ~Words() {
+            if (p) cudaFreeHost(p);
+        }
+    };
+    static thread_local Words w;
+    if (!w.p && cudaHostAlloc(reinterpret_cast<void **>(&w.p), kEndWords * sizeof(unsigned), cudaHostAllocPortable) !=
+                    cudaSuccess) {
+        cudaGetLastError();
+        w.p = nullptr;
+    }
+    return w.p;
+}
+
+// A stream's status words, and the range verdict of an FP64 run (state, may be
+// NULL), once the stream has drained.
+struct RunEnd {
+    bool read = false;
+    unsigned status[kStatusWords] = {};
+    int state = 0;
+};
+static int read_end(const unsigned *w, const int *state, cudaStream_t st, RunEnd *end) {
+    unsigned local[kEndWords], *h = pinned_end_words();
+    if (!h) h = local;
+    cudaError_t e = cudaMemcpyAsync(h, w, sizeof end->status, cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess && state)
+        e = cudaMemcpyAsync(h + kStatusWords, state, sizeof *state, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return cuda_error(e, "device status read");
+    std::memcpy(end->status, h, sizeof end->status);
+    if (state) std::memcpy(&end->state, h + kStatusWords, sizeof end->state);
+    end->read = true;
+    return UHS_OK;
+}
+
+// Report and clear what a drained stream's status words hold.
+static int report_status(unsigned *w, const unsigned *h, cudaStream_t st) {
     if (!h[0]) return UHS_OK;
-    cudaMemsetAsync(w, 0, sizeof h, st);
+    cudaMemsetAsync(w, 0, kStatusWords * sizeof(unsigned), st);
     cudaStreamSynchronize(st);
     if (h[0] & kDevErrTimeout)
         return set_error(UHS_ETIMEOUT,
@@ -1042,17 +1078,24 @@ static int check_status_word(unsigned *w, cudaStream_t st) {
                                  "run this grid with UHS_ARITH_FMA");
 }
 
-static int check_device_errors(cudaStream_t st) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    return check_status_word(stream_error_word(dev, st), st);
+static int check_status_word(unsigned *w, cudaStream_t st) {
+    if (!w) return UHS_OK;
+    RunEnd end;
+    const int rc = read_end(w, nullptr, st, &end);
+    return rc ? rc : report_status(w, end.status, st);
 }
 
-static int finish(const uhs_params *p, cudaStream_t st) {
+// The end of a call: wait for the stream and report its status, which *end may
+// hold already.
+static int finish(const uhs_params *p, cudaStream_t st, const RunEnd *end = nullptr) {
     if (p && (p->flags & UHS_FLAG_NO_SYNC)) return UHS_OK;
-    cudaError_t e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) return cuda_error(e, "stream synchronise");
-    return check_device_errors(st);
+    int dev = 0;
+    cudaGetDevice(&dev);
+    unsigned *w = stream_error_word(dev, st);
+    if (end && end->read) return report_status(w, end->status, st);
+    if (w) return check_status_word(w, st);
+    const cudaError_t e = cudaStreamSynchronize(st);
+    return e == cudaSuccess ? UHS_OK : cuda_error(e, "stream synchronise");
 }
 
 static int prepare(const uhs_stencil_desc *d, const uhs_memref *a, const uhs_memref *b, GridView *va,
@@ -1688,27 +1731,16 @@ static cudaError_t dev_alloc_async(void **p, size_t bytes, cudaStream_t st) {
     return e;
 }
 
-// The device's verdict on an FP64 run's range, once its stream has drained.
-static int read_verdict(const int *state, cudaStream_t st, bool *native) {
-    int v = 0;
-    cudaError_t e = cudaMemcpyAsync(&v, state, sizeof v, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) return cuda_error(e, "range verdict");
-    *native = v == kRunNative;
-    return UHS_OK;
-}
-
 // A run held in shared memory from its first sweep to its last (resident.cuh):
 // rank-2 star and box programs of two or more sweeps on FP64 (UHS_ARITH_AUTO) and
 // FP32 grids whose domain fits, when the caller and the tuner database leave
 // the launch to the backend.  *ran stays false when it does not apply, or
 // its scratch or its launch could not be had, and the sweeps are launched one
-// by one; with *native set, the data's range needs native FP64 arithmetic
-// (both grids are then as they were).
+// by one.  FP64: *end is read; with its state kRunNative the data's range needs
+// native FP64 arithmetic (both grids are then as they were).
 static int run_resident(const SweepSpec &sp, const Plan &pl, const uhs_params *p, const GridView &va,
-                        const GridView &vb, int T, cudaStream_t st, bool *ran, bool *native) {
+                        const GridView &vb, int T, cudaStream_t st, bool *ran, RunEnd *end) {
     *ran = false;
-    *native = false;
     const bool f64 = pl.st == kStF64;
     const int other = UHS_FLAG_IN_PLACE | UHS_FLAG_XSHUFFLE;
     // FP64 from two sweeps on (the range scan and the conversions go too: 256^2
@@ -1764,7 +1796,7 @@ static int run_resident(const SweepSpec &sp, const Plan &pl, const uhs_params *p
         return UHS_OK;
     }
     *ran = true;
-    const int rc = f64 ? read_verdict(c.verdict, st, native) : UHS_OK;
+    const int rc = f64 ? read_end(err, c.verdict, st, end) : UHS_OK;
     cudaFreeAsync(buf, st);
     return rc;
 }
@@ -1808,9 +1840,8 @@ static GridView shifted_view(const GridView &g, const int64_t from[3], const int
 // 87 -> 95).  2D rows that cannot load in 8-byte pairs: 3000 x 3001 21.9 -> 19.3
 // us a sweep.
 static int run_on_copies(const SweepSpec &sp, const Plan &pl, const uhs_params *p, const GridView &va,
-                         const GridView &vb, int T, cudaStream_t st, bool *ran, bool *native) {
+                         const GridView &vb, int T, cudaStream_t st, bool *ran, RunEnd *end) {
     *ran = false;
-    *native = false;
     const bool f64 = pl.st == kStF64, is2d = sp.rank == 2;
     const int R = pl.R;
     if (T < 4 || pl.kernel != UHS_KERNEL_STREAM || pl.cfg.k_temporal > 1 || pl.cfg.use_tma < 0 ||
@@ -1909,7 +1940,7 @@ static int run_on_copies(const SweepSpec &sp, const Plan &pl, const uhs_params *
     if (!rc) rc = l_b.launch();
     if (!rc) rc = l_a.launch();
     if (f64) {
-        const int vrc = read_verdict(&run->state, st, native);
+        const int vrc = read_end(err, &run->state, st, end);
         if (!rc) rc = vrc;
     }
     cudaFreeAsync(buf, st);
@@ -1921,9 +1952,8 @@ static int run_on_copies(const SweepSpec &sp, const Plan &pl, const uhs_params *
 // sweeps follow it, and the host learns of it at the end.  *ran stays false
 // when the word for the verdict cannot be had.
 static int run_in_place_scanned(const SweepSpec &sp, const Plan &pl, const GridView &va, const GridView &vb, int T,
-                                cudaStream_t st, bool *ran, bool *native) {
+                                cudaStream_t st, bool *ran, RunEnd *end) {
     *ran = false;
-    *native = false;
     if (!pl.auto_df32 || pl.kernel != UHS_KERNEL_STREAM || pl.cfg.k_temporal > 1) return UHS_OK;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) {
@@ -1954,7 +1984,7 @@ static int run_in_place_scanned(const SweepSpec &sp, const Plan &pl, const GridV
         launch_run_scan(va, T > 1 ? &vb : nullptr, sp.lb, sp.ub, reach, run_growth(sp, T), err + kRunCtlWord, run, st);
     if (e != cudaSuccess) rc = cuda_error(e, "range scan");
     for (int t = 0; t < std::max(T, 1) && !rc; ++t) rc = (t % 2 ? ba : ab).launch();
-    const int vrc = read_verdict(&run->state, st, native);
+    const int vrc = read_end(err, &run->state, st, end);
     cudaFreeAsync(buf, st);
     return rc ? rc : vrc;
 }
@@ -2210,9 +2240,11 @@ int uhs_sweep(const uhs_stencil_desc *d, const uhs_memref *in, const uhs_memref 
     Plan pl;
     if ((rc = plan_sweep(sp, p, vi, &pl))) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    bool done = false, native = false;
-    if ((rc = run_in_place_scanned(sp, pl, vi, vo, 1, st, &done, &native))) return rc;
-    if (done && !native) return finish(p, st);
+    bool done = false;
+    RunEnd end;
+    if ((rc = run_in_place_scanned(sp, pl, vi, vo, 1, st, &done, &end))) return rc;
+    const bool native = end.state == kRunNative;
+    if (done && !native) return finish(p, st, &end);
     if (pl.auto_df32 && (native || !range_ok(sp, vi, vo, 1, st, &pl.pair_shift))) {
         fall_back_native(pl);
     }
@@ -2234,13 +2266,15 @@ int uhs_run(const uhs_stencil_desc *d, const uhs_memref *a, const uhs_memref *b,
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     // on chip, on the library's copies, or in place under the device's range
     // verdict; a run whose range needs native FP64 has left the grids as they were
-    bool done = false, native = false;
-    if ((rc = run_resident(sp, pl, p, va, vb, d->iterations, st, &done, &native))) return rc;
-    if (!done && (rc = run_on_copies(sp, pl, p, va, vb, d->iterations, st, &done, &native))) return rc;
+    bool done = false;
+    RunEnd end;
+    if ((rc = run_resident(sp, pl, p, va, vb, d->iterations, st, &done, &end))) return rc;
+    if (!done && (rc = run_on_copies(sp, pl, p, va, vb, d->iterations, st, &done, &end))) return rc;
     if (!done && d->iterations > 0 && !pair_eligible(pl, d->iterations, p) &&
-        (rc = run_in_place_scanned(sp, pl, va, vb, d->iterations, st, &done, &native)))
+        (rc = run_in_place_scanned(sp, pl, va, vb, d->iterations, st, &done, &end)))
         return rc;
-    if (done && !native) return finish(p, st);
+    const bool native = end.state == kRunNative;
+    if (done && !native) return finish(p, st, &end);
     if (pl.auto_df32 && d->iterations > 0 &&
         (native || !range_ok(sp, va, vb, d->iterations, st, &pl.pair_shift))) {
         fall_back_native(pl);
@@ -2307,8 +2341,6 @@ int uhs_batch_run(uhs_batch *batch, void *stream, int32_t flags) {
         count_launch(static_cast<int>(batch->impl->launches));
     }
     if (flags & UHS_FLAG_NO_SYNC) return UHS_OK;
-    cudaError_t e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) return cuda_error(e, "stream synchronise");
     return check_status_word(batch->impl->d_status, st);
 }
 

@@ -10,6 +10,7 @@ from __future__ import annotations
 
 import ctypes
 import itertools
+import struct
 from dataclasses import dataclass, field, replace
 from typing import Sequence
 
@@ -80,9 +81,15 @@ class DescHolder:
 
     def __init__(self, s: Stencil):
         n = s.nterms
-        self.terms = (_lib.Term * n)()
-        for i, (dz, dy, dx, c) in enumerate(s.terms):
-            self.terms[i] = _lib.Term(dz, dy, dx, s.param_terms.get(i, -1), float(c))
+        # one pack of all terms: field by field, a 343-term box took 180 us, most
+        # of a short run
+        flat = []
+        for t in s.terms:
+            flat += (t[0], t[1], t[2], -1, t[3])
+        for i, k in s.param_terms.items():
+            if 0 <= i < n:
+                flat[5 * i + 3] = k
+        self.terms = (_lib.Term * n).from_buffer_copy(struct.pack("=" + "iiiid" * n, *flat))
         self.params = (ctypes.c_double * max(1, len(s.params)))(*s.params) if s.params else None
         self.desc = _lib.StencilDesc()
         self.desc.rank = s.rank
