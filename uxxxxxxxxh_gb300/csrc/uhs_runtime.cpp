@@ -573,9 +573,11 @@ static int plan_sweep(const SweepSpec &sp, const uhs_params *p, const GridView &
     // tile_z overrides it.
     if (!is2d) {
         const bool df = arith == UHS_ARITH_DF32, f32 = sp.dtype == UHS_F32 && !df;
-        // (float-pair 3d1r star with bounded sums: 374 vs 363 GStencil/s at 16 planes)
+        // (float-pair 3d1r star: 8 planes, us at 512^3 8 / 16 planes 315 / 335 on
+        // whole lines, 325 / 361 off them; longer chunks of its HBM-bound sweep
+        // keep more planes of neighbouring tiles apart in L2)
         // (FP64 grids swept in place: 64 planes)
-        if (shape == kStar3) pl->zcap = df ? ((R >= 2 || sp.dtype == UHS_F64) ? 64 : 16) : f32 ? (R == 3 ? 64 : 16) : 0;
+        if (shape == kStar3) pl->zcap = df ? ((R >= 2 || sp.dtype == UHS_F64) ? 64 : 8) : f32 ? (R == 3 ? 64 : 16) : 0;
         else if (sep) pl->zcap = (df || f32) ? (R >= 2 ? 64 : f32 ? 16 : 0) : 0;
         else pl->zcap = df ? (R >= 2 ? 16 : 64) : f32 ? (R >= 2 ? 64 : 0) : 0;
     }
@@ -600,6 +602,9 @@ static int plan_sweep(const SweepSpec &sp, const uhs_params *p, const GridView &
     if (cfg.use_tma > 0 && !tma_ok)
         return set_error(UHS_EUNSUPPORTED, "TMA needs 16-byte aligned grids and row/plane strides");
     pl->ld = tma_ok ? kLdTma : kLdCpAsync;
+    // FP32 3d1r star by TMA: 10 planes, 169 vs 177 us at 512^3 and 16 (by
+    // cp.async 16, 209 vs 210; odd rows 68 vs 71 at 300 x 301 x 301)
+    if (shape == kStar3 && R == 1 && sp.dtype == UHS_F32 && tma_ok) pl->zcap = 10;
     if (sep) {
         pl->shape = shape = (shape == kBox3) ? kSep3 : kSep2;
         pl->coef = fac;
@@ -793,6 +798,10 @@ static int stream_zchunk(const SweepSpec &sp, const Plan &pl, const StreamCall &
         if (sp.rank == 2 && c.ar == kArDf32 && tiles * ((nz + 15) / 16) >= 2 * slots)
             floor_z = std::max(16, 4 * c.R);
         zchunk = static_cast<int>(std::max<int64_t>(floor_z, (nz + chunks - 1) / chunks));
+        // Float-pair grids of a 2d1r star in four waves or more of 16 rows: 161.5
+        // vs 167.0 us at 8192^2 and 36 rows (four waves)
+        if (c.shape == kStar2 && c.R == 1 && c.st == kStF32x2 && tiles * ((nz + 15) / 16) >= 4 * slots)
+            zchunk = std::min(zchunk, 16);
         if (pl.zcap > 0) zchunk = std::min(zchunk, std::max(pl.zcap, floor_z));
         // Grids below the waves that rule is made for: shorter chunks where
         // the estimate says at least 3 % (us per sweep at the rule's chunk ->
