@@ -617,14 +617,18 @@ __device__ __forceinline__ bool stream_item(const Args &a, int bxi, int byi, int
     int s_iss = PD % NSTG;
     int s_cmp = 0;  // compute-ring slot of plane j
     // 2R+1 copies of the plane step, the length of the z-queue, so its shifts
-    // become register renaming: 2D stars and separable boxes, and 3D radius-1
-    // stars.  GB300, GStencil/s: 3d7pt float pairs 175.4 -> 179.8, 2d5pt
-    // 176.4 -> 182.3 (FP32 490 -> 511); at 8192^2 2d9pt 145.6 -> 153.8 (FP32
-    // 544 -> 587), 2d13pt 110.3 -> 124.5 (FP32 479 -> 521), separable 2D
-    // boxes r1/r2/r3 +4/+14/+8 %.  3D stars of radius 2-3, whose loop bodies
-    // are several times larger, lose (3d13pt 118.5 -> 94.4), and so does the
-    // separable 3D r1 box (148.0 -> 145.6).
-    constexpr int UNROLL_Q = ((STAR && R == 1) || ((STAR || SEP) && IS2D)) ? 2 * R + 1 : 1;
+    // become register renaming: 2D stars and separable boxes, 3D stars of
+    // radius 1, of radius 2 on float-pair and FP32 grids, of radius 3 on FP32.  GB300, GStencil/s: 3d7pt float
+    // pairs 175.4 -> 179.8, 2d5pt 176.4 -> 182.3 (FP32 490 -> 511); at 8192^2
+    // 2d9pt 145.6 -> 153.8 (FP32 544 -> 587), 2d13pt 110.3 -> 124.5 (FP32 479 ->
+    // 521), separable 2D boxes r1/r2/r3 +4/+14/+8 % (all with the sums of 12
+    // operations a term); us at 512^3: 3d13pt float pairs 478 -> 467, FP32 195 ->
+    // 189, 3d19pt FP32 229 -> 195.  Float pairs of radius 3, whose loop body is
+    // seven times 20 KB then, lose (676 -> 922), and so do FP64 grids in place
+    // (radius 2 442 -> 452 at 384^3) and the separable 3D r1 box (148.0 -> 145.6
+    // GStencil/s).
+    constexpr bool UNROLL_STAR = R == 1 || (R == 2 && C::ST != kStF64) || C::ST == kStF32;
+    constexpr int UNROLL_Q = (STAR && UNROLL_STAR) || ((STAR || SEP) && IS2D) ? 2 * R + 1 : 1;
 #pragma unroll UNROLL_Q
     for (int j = 0; j < nq; ++j) {
         bool ok = true;
