@@ -626,9 +626,15 @@ __device__ __forceinline__ bool stream_item(const Args &a, int bxi, int byi, int
     // 189, 3d19pt FP32 229 -> 195.  Float pairs of radius 3, whose loop body is
     // seven times 20 KB then, lose (676 -> 922), and so do FP64 grids in place
     // (radius 2 442 -> 452 at 384^3) and the separable 3D r1 box (148.0 -> 145.6
-    // GStencil/s).
+    // GStencil/s).  Two copies, which halve the moves, where 2R+1 are too many: us
+    // at 384^3 3d19pt float pairs 305 -> 294; separable 3D r1 / r2 float pairs 193 /
+    // 341 -> 189 / 337, FP32 r2 / r3 113 / 216 -> 108 / 196 (FP64 in place 19 points
+    // 562 -> 599, separable float pairs r3 531 -> 533: one copy).
     constexpr bool UNROLL_STAR = R == 1 || (R == 2 && C::ST != kStF64) || C::ST == kStF32;
-    constexpr int UNROLL_Q = (STAR && UNROLL_STAR) || ((STAR || SEP) && IS2D) ? 2 * R + 1 : 1;
+    constexpr bool NATIVE64 = C::ST == kStF64 && C::AR == kArNative;
+    constexpr bool TWICE = !IS2D && !NATIVE64 &&
+                           ((STAR && C::ST == kStF32x2) || (SEP && (R <= 2 || C::ST == kStF32)));
+    constexpr int UNROLL_Q = (STAR && UNROLL_STAR) || ((STAR || SEP) && IS2D) ? 2 * R + 1 : TWICE ? 2 : 1;
 #pragma unroll UNROLL_Q
     for (int j = 0; j < nq; ++j) {
         bool ok = true;
