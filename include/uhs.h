@@ -58,8 +58,8 @@ enum {
     UHS_ARITH_AUTO = 0,  /* the backend picks: for F64 grids on the streaming kernel,
                             float pairs scaled by a power of two chosen by a device
                             scan of the cells the program reads (one extra read of a;
-                            the call waits for its verdict, also with
-                            UHS_FLAG_NO_SYNC), unless they hold Inf/NaN
+                            with UHS_FLAG_NO_SYNC the call still waits for
+                            that scan), unless they hold Inf/NaN
                             or span more than about 2^169 between the largest
                             magnitude grown by (sum|c|)^T and the smallest nonzero
                             one; then UHS_ARITH_FMA */
@@ -187,8 +187,8 @@ int uhs_validate(const uhs_stencil_desc *desc, const uhs_memref *a, const uhs_me
  * stream has drained, which is what the reference's entry does.
  *
  * Resident runs: rank-2 star and box programs whose domain fits in the GPU's
- * shared memory (FP64 under UHS_ARITH_AUTO from two sweeps on, FP32 from
- * eight), with the launch left to the backend (params NULL or all zero apart
+ * shared memory (FP64 under UHS_ARITH_AUTO from two sweeps on, without
+ * UHS_FLAG_NO_SYNC; FP32 from eight), with the launch left to the backend (params NULL or all zero apart
  * from flags, no tuner-database entry), run in one cooperative launch that
  * holds the grid on chip from the first sweep to the last and writes both
  * grids at its end.  Results are bit-identical to the sweeps launched one by

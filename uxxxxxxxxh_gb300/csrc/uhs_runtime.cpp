@@ -1073,6 +1073,31 @@ static int read_end(const unsigned *w, const int *state, cudaStream_t st, RunEnd
     return UHS_OK;
 }
 
+// The range verdict of a call that does not wait for its stream
+// (UHS_FLAG_NO_SYNC): copied right behind the scan, waited for alone while the
+// sweeps enqueued after it run on.
+struct EarlyVerdict {
+    cudaEvent_t ev = nullptr;
+    unsigned local = 0, *h = nullptr;
+    ~EarlyVerdict() {
+        if (ev) cudaEventDestroy(ev);
+    }
+    cudaError_t enqueue(const int *state, cudaStream_t st) {
+        h = pinned_end_words();
+        if (!h) h = &local;
+        cudaError_t e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(h, state, sizeof *h, cudaMemcpyDeviceToHost, st);
+        return e == cudaSuccess ? cudaEventRecord(ev, st) : e;
+    }
+    int wait(RunEnd *end) {
+        const cudaError_t e = cudaEventSynchronize(ev);
+        if (e != cudaSuccess) return cuda_error(e, "range verdict");
+        end->state = static_cast<int>(*h);
+        return UHS_OK;
+    }
+};
+static bool waits(const uhs_params *p) { return !(p && (p->flags & UHS_FLAG_NO_SYNC)); }
+
 // Report and clear what a drained stream's status words hold.
 static int report_status(unsigned *w, const unsigned *h, cudaStream_t st) {
     if (!h[0]) return UHS_OK;
@@ -1756,8 +1781,8 @@ static int run_resident(const SweepSpec &sp, const Plan &pl, const uhs_params *p
     // to 1448^2, T = 4, 70-110 us a run against 95-150); FP32 from eight: at T
     // = 4 its set-up costs what the launches do (48-83 against 45-75 us).
     if (T < (f64 ? 2 : 8) || sp.rank != 2 || pl.kernel != UHS_KERNEL_STREAM || !params_are_auto(p) || (p && (p->flags & other)) ||
-        (f64 ? !pl.auto_df32 : pl.st != kStF32))
-        return UHS_OK;
+        (f64 ? !pl.auto_df32 || !waits(p) : pl.st != kStF32))
+        return UHS_OK;  // (FP64 without a wait: the verdict would come with the launch's end)
     const int64_t nz = sp.ub[1] - sp.lb[1], nx = sp.ub[2] - sp.lb[2];
     const int cell = f64 ? 8 : 4;
     const ResPlan rp = plan_resident(pl.shape != kStar2, pl.R, cell, static_cast<int>(pl.coef.size()), nz, nx,
@@ -1936,9 +1961,11 @@ static int run_on_copies(const SweepSpec &sp, const Plan &pl, const uhs_params *
     *ran = true;
     int rc = UHS_OK;
     cudaError_t e = cudaSuccess;
+    EarlyVerdict early;
     if (f64) {
         l_b.c.out2 = kernel_view(sp2, pb);
         e = launch_run_scan(va, &vb, sp.lb, sp.ub, reach, run_growth(sp, T), err + kRunCtlWord, run, st);
+        if (e == cudaSuccess && !waits(p)) e = early.enqueue(&run->state, st);
     }
     if (e == cudaSuccess) e = launch_shell_copy(f64, va, vb, pa, pb, sp.lb, sp.ub, clb, reach, run, st);
     if (e != cudaSuccess) rc = cuda_error(e, "run set-up");
@@ -1949,7 +1976,7 @@ static int run_on_copies(const SweepSpec &sp, const Plan &pl, const uhs_params *
     if (!rc) rc = l_b.launch();
     if (!rc) rc = l_a.launch();
     if (f64) {
-        const int vrc = read_end(err, &run->state, st, end);
+        const int vrc = rc ? rc : waits(p) ? read_end(err, &run->state, st, end) : early.wait(end);
         if (!rc) rc = vrc;
     }
     cudaFreeAsync(buf, st);
@@ -1960,8 +1987,8 @@ static int run_on_copies(const SweepSpec &sp, const Plan &pl, const uhs_params *
 // b's shell is not read then): the range scan decides on the device, the
 // sweeps follow it, and the host learns of it at the end.  *ran stays false
 // when the word for the verdict cannot be had.
-static int run_in_place_scanned(const SweepSpec &sp, const Plan &pl, const GridView &va, const GridView &vb, int T,
-                                cudaStream_t st, bool *ran, RunEnd *end) {
+static int run_in_place_scanned(const SweepSpec &sp, const Plan &pl, const uhs_params *p, const GridView &va,
+                                const GridView &vb, int T, cudaStream_t st, bool *ran, RunEnd *end) {
     *ran = false;
     if (!pl.auto_df32 || pl.kernel != UHS_KERNEL_STREAM || pl.cfg.k_temporal > 1) return UHS_OK;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
@@ -1989,13 +2016,15 @@ static int run_in_place_scanned(const SweepSpec &sp, const Plan &pl, const GridV
         return rc;
     }
     *ran = true;
-    const cudaError_t e =
+    cudaError_t e =
         launch_run_scan(va, T > 1 ? &vb : nullptr, sp.lb, sp.ub, reach, run_growth(sp, T), err + kRunCtlWord, run, st);
+    EarlyVerdict early;
+    if (e == cudaSuccess && !waits(p)) e = early.enqueue(&run->state, st);
     if (e != cudaSuccess) rc = cuda_error(e, "range scan");
     for (int t = 0; t < std::max(T, 1) && !rc; ++t) rc = (t % 2 ? ba : ab).launch();
-    const int vrc = read_end(err, &run->state, st, end);
+    if (!rc) rc = waits(p) ? read_end(err, &run->state, st, end) : early.wait(end);
     cudaFreeAsync(buf, st);
-    return rc ? rc : vrc;
+    return rc;
 }
 
 // Pair-resident run of a float-pair FP64 program (see uhs_run in uhs.h):
@@ -2251,7 +2280,7 @@ int uhs_sweep(const uhs_stencil_desc *d, const uhs_memref *in, const uhs_memref 
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     bool done = false;
     RunEnd end;
-    if ((rc = run_in_place_scanned(sp, pl, vi, vo, 1, st, &done, &end))) return rc;
+    if ((rc = run_in_place_scanned(sp, pl, p, vi, vo, 1, st, &done, &end))) return rc;
     const bool native = end.state == kRunNative;
     if (done && !native) return finish(p, st, &end);
     if (pl.auto_df32 && (native || !range_ok(sp, vi, vo, 1, st, &pl.pair_shift))) {
@@ -2280,7 +2309,7 @@ int uhs_run(const uhs_stencil_desc *d, const uhs_memref *a, const uhs_memref *b,
     if ((rc = run_resident(sp, pl, p, va, vb, d->iterations, st, &done, &end))) return rc;
     if (!done && (rc = run_on_copies(sp, pl, p, va, vb, d->iterations, st, &done, &end))) return rc;
     if (!done && d->iterations > 0 && !pair_eligible(pl, d->iterations, p) &&
-        (rc = run_in_place_scanned(sp, pl, va, vb, d->iterations, st, &done, &end)))
+        (rc = run_in_place_scanned(sp, pl, p, va, vb, d->iterations, st, &done, &end)))
         return rc;
     const bool native = end.state == kRunNative;
     if (done && !native) return finish(p, st, &end);
