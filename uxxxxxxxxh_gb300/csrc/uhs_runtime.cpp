@@ -1096,6 +1096,13 @@ struct EarlyVerdict {
         return UHS_OK;
     }
 };
+// Whether the domain's corners fit the 32-bit coordinates of the kernels that
+// walk shells and boxes.
+static bool small_coordinates(const SweepSpec &sp) {
+    for (int i = 0; i < 3; ++i)
+        if (sp.ub[i] >= (int64_t(1) << 30)) return false;
+    return true;
+}
 static bool waits(const uhs_params *p) { return !(p && (p->flags & UHS_FLAG_NO_SYNC)); }
 
 // Report and clear what a drained stream's status words hold.
@@ -1781,7 +1788,7 @@ static int run_resident(const SweepSpec &sp, const Plan &pl, const uhs_params *p
     // to 1448^2, T = 4, 70-110 us a run against 95-150); FP32 from eight: at T
     // = 4 its set-up costs what the launches do (48-83 against 45-75 us).
     if (T < (f64 ? 2 : 8) || sp.rank != 2 || pl.kernel != UHS_KERNEL_STREAM || !params_are_auto(p) || (p && (p->flags & other)) ||
-        (f64 ? !pl.auto_df32 || !waits(p) : pl.st != kStF32))
+        (f64 ? !pl.auto_df32 || !waits(p) : pl.st != kStF32) || !small_coordinates(sp))
         return UHS_OK;  // (FP64 without a wait: the verdict would come with the launch's end)
     const int64_t nz = sp.ub[1] - sp.lb[1], nx = sp.ub[2] - sp.lb[2];
     const int cell = f64 ? 8 : 4;
@@ -1879,7 +1886,7 @@ static int run_on_copies(const SweepSpec &sp, const Plan &pl, const uhs_params *
     const bool f64 = pl.st == kStF64, is2d = sp.rank == 2;
     const int R = pl.R;
     if (T < 4 || pl.kernel != UHS_KERNEL_STREAM || pl.cfg.k_temporal > 1 || pl.cfg.use_tma < 0 ||
-        (p && (p->flags & UHS_FLAG_IN_PLACE)) || (pl.shape == kBox3 && R >= 2))
+        (p && (p->flags & UHS_FLAG_IN_PLACE)) || (pl.shape == kBox3 && R >= 2) || !small_coordinates(sp))
         return UHS_OK;
     int64_t n[3], points = 1;
     for (int i = 0; i < 3; ++i) points *= n[i] = sp.ub[i] - sp.lb[i];
@@ -1990,7 +1997,8 @@ static int run_on_copies(const SweepSpec &sp, const Plan &pl, const uhs_params *
 static int run_in_place_scanned(const SweepSpec &sp, const Plan &pl, const uhs_params *p, const GridView &va,
                                 const GridView &vb, int T, cudaStream_t st, bool *ran, RunEnd *end) {
     *ran = false;
-    if (!pl.auto_df32 || pl.kernel != UHS_KERNEL_STREAM || pl.cfg.k_temporal > 1) return UHS_OK;
+    if (!pl.auto_df32 || pl.kernel != UHS_KERNEL_STREAM || pl.cfg.k_temporal > 1 || !small_coordinates(sp))
+        return UHS_OK;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) {
         cudaGetLastError();
