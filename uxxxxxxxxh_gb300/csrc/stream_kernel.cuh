@@ -592,7 +592,12 @@ __device__ __forceinline__ bool stream_item(const Args &a, int bxi, int byi, int
     // df32.cuh).
     constexpr bool PACK = C::PACKED && !std::is_same_v<Args, BatchArgs>;
     constexpr int NPR = PACK ? NPT / 2 : 1;
+    // a result outside the float range; a loaded cell outside it.  A run whose
+    // range was scanned on the device reports results alone: the scan has
+    // bounded every cell that its sums read, and a tile's other cells (past the
+    // radius, in the caller's grid) may hold anything
     unsigned range_err = 0;
+    [[maybe_unused]] unsigned load_err = 0;
     const bool x_ok = x0 + VX * tx < a.ub2;
     // output pointer of (zs, y0 + ty*VY, x0 + VX*tx); points vmin..vmax-1
     // are written: rows beyond ub1 are masked, and with two points along x
@@ -675,7 +680,7 @@ __device__ __forceinline__ bool stream_item(const Args &a, int bxi, int byi, int
 #pragma unroll
                     for (int c0 = 0; c0 < WL; c0 += BX)
                         if (c0 + tx < WL)
-                            dp[r * W + c0 + tx] = split_f64(sp[r * W + c0 + tx], range_err, bias);
+                            dp[r * W + c0 + tx] = split_f64(sp[r * W + c0 + tx], load_err, bias);
                 }
             }
             __syncthreads();
@@ -1119,6 +1124,10 @@ __device__ __forceinline__ bool stream_item(const Args &a, int bxi, int byi, int
         if (s_stg == 0) phase ^= 1u;
         s_iss = s_iss + 1 == NSTG ? 0 : s_iss + 1;
         if constexpr (C::CONVERT) s_cmp = s_cmp + 1 == NCMP ? 0 : s_cmp + 1;
+    }
+    if constexpr (C::CONVERT) {
+        if constexpr (!std::is_same_v<Args, BatchArgs>) load_err = a.run ? 0u : load_err;
+        range_err |= load_err;
     }
     if constexpr (C::CONVERT || C::JOIN) {
         if (range_err) atomicOr(a.err, kDevErrRange);
