@@ -193,8 +193,8 @@ int uhs_validate(const uhs_stencil_desc *desc, const uhs_memref *a, const uhs_me
  * holds the grid on chip from the first sweep to the last and writes both
  * grids at its end.  Results are bit-identical to the sweeps launched one by
  * one.  Scratch: two words per cell from the library's pool; without it, on a
- * capturing stream, or with UHS_FLAG_IN_PLACE, the sweeps are launched one by
- * one.  The kernel makes UHS_ARITH_AUTO's range check itself, over the cells
+ * capturing stream, with UHS_FLAG_IN_PLACE, or on cudaStreamPerThread with
+ * UHS_FLAG_NO_SYNC, the sweeps are launched one by one.  The kernel makes UHS_ARITH_AUTO's range check itself, over the cells
  * the program reads.
  *
  * Pair-resident runs: FP64 grids swept in float-pair arithmetic (UHS_ARITH_AUTO

@@ -27,6 +27,7 @@
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <thread>
 #include <vector>
 
 namespace uhs {
@@ -72,12 +73,15 @@ static int cuda_error(cudaError_t e, const char *what) {
 // Status words (kStatusWords x unsigned, layout in uhs_kernels.h) in device
 // memory, one per (device, stream), allocated at first use and kept for the
 // process.  Calls on different streams (or host threads with their own streams) never
-// share a word, so one call's errors and scan results cannot leak into
-// another's.
+// share a word, so one call's errors and scan results, and the counters its
+// kernels meet at, cannot leak into another's.  cudaStreamPerThread is one
+// handle for a stream of each host thread's own, so there the thread counts too
+// (by its id, which the system gives to a later thread again: outlives_thread).
 unsigned *stream_error_word(int device, cudaStream_t stream) {
     static std::mutex mu;
-    static std::map<std::pair<int, uintptr_t>, unsigned *> words;
-    const auto key = std::make_pair(device, reinterpret_cast<uintptr_t>(stream));
+    static std::map<std::tuple<int, uintptr_t, std::thread::id>, unsigned *> words;
+    const auto key = std::make_tuple(device, reinterpret_cast<uintptr_t>(stream),
+                                     stream == cudaStreamPerThread ? std::this_thread::get_id() : std::thread::id());
     std::lock_guard<std::mutex> lk(mu);
     auto it = words.find(key);
     if (it != words.end()) return it->second;
@@ -1053,18 +1057,21 @@ static unsigned *pinned_end_words() {
 }
 
 // A stream's status words, and the range verdict of an FP64 run (state, may be
-// NULL), once the stream has drained.
+// NULL), once the stream has drained.  scratch (may be NULL, may hold the
+// verdict) is freed on the stream ahead of the wait, so that nothing of a call
+// that waits is pending when it returns.
 struct RunEnd {
     bool read = false;
     unsigned status[kStatusWords] = {};
     int state = 0;
 };
-static int read_end(const unsigned *w, const int *state, cudaStream_t st, RunEnd *end) {
+static int read_end(const unsigned *w, const int *state, cudaStream_t st, RunEnd *end, void *scratch = nullptr) {
     unsigned local[kEndWords], *h = pinned_end_words();
     if (!h) h = local;
     cudaError_t e = cudaMemcpyAsync(h, w, sizeof end->status, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess && state)
         e = cudaMemcpyAsync(h + kStatusWords, state, sizeof *state, cudaMemcpyDeviceToHost, st);
+    if (scratch) cudaFreeAsync(scratch, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return cuda_error(e, "device status read");
     std::memcpy(end->status, h, sizeof end->status);
@@ -1104,6 +1111,12 @@ static bool small_coordinates(const SweepSpec &sp) {
     return true;
 }
 static bool waits(const uhs_params *p) { return !(p && (p->flags & UHS_FLAG_NO_SYNC)); }
+// Whether the thread may end before the call's work has: its own stream, and no
+// wait.  Kernels that meet at the stream's words (a later thread with this
+// thread's id takes them over) and stream-ordered scratch are kept off such
+// calls: their ranges are scanned under a host wait and their sweeps launched
+// one by one on the caller's grids (pair-resident runs as ever).
+static bool outlives_thread(const uhs_params *p, cudaStream_t st) { return st == cudaStreamPerThread && !waits(p); }
 
 // Report and clear what a drained stream's status words hold.
 static int report_status(unsigned *w, const unsigned *h, cudaStream_t st) {
@@ -1137,6 +1150,14 @@ static int finish(const uhs_params *p, cudaStream_t st, const RunEnd *end = null
     if (w) return check_status_word(w, st);
     const cudaError_t e = cudaStreamSynchronize(st);
     return e == cudaSuccess ? UHS_OK : cuda_error(e, "stream synchronise");
+}
+
+// The end of a call that ran in float pairs or FP32 by a route of its own.
+// scanned: its kernels followed a range verdict, which must then be the pairs'.
+static int finish_run(const uhs_params *p, cudaStream_t st, const RunEnd &end, bool scanned) {
+    const int rc = finish(p, st, &end);
+    if (rc || !scanned || end.state == kRunPairs) return rc;
+    return set_error(UHS_ECUDA, "the run's range scan left no verdict (%d)", end.state);
 }
 
 static int prepare(const uhs_stencil_desc *d, const uhs_memref *a, const uhs_memref *b, GridView *va,
@@ -1788,7 +1809,7 @@ static int run_resident(const SweepSpec &sp, const Plan &pl, const uhs_params *p
     // to 1448^2, T = 4, 70-110 us a run against 95-150); FP32 from eight: at T
     // = 4 its set-up costs what the launches do (48-83 against 45-75 us).
     if (T < (f64 ? 2 : 8) || sp.rank != 2 || pl.kernel != UHS_KERNEL_STREAM || !params_are_auto(p) || (p && (p->flags & other)) ||
-        (f64 ? !pl.auto_df32 || !waits(p) : pl.st != kStF32) || !small_coordinates(sp))
+        (f64 ? !pl.auto_df32 || !waits(p) : pl.st != kStF32) || !small_coordinates(sp) || outlives_thread(p, st))
         return UHS_OK;  // (FP64 without a wait: the verdict would come with the launch's end)
     const int64_t nz = sp.ub[1] - sp.lb[1], nx = sp.ub[2] - sp.lb[2];
     const int cell = f64 ? 8 : 4;
@@ -1837,9 +1858,9 @@ static int run_resident(const SweepSpec &sp, const Plan &pl, const uhs_params *p
         return UHS_OK;
     }
     *ran = true;
-    const int rc = f64 ? read_end(err, c.verdict, st, end) : UHS_OK;
+    if (f64) return read_end(err, c.verdict, st, end, buf);
     cudaFreeAsync(buf, st);
-    return rc;
+    return UHS_OK;
 }
 
 // Elements from one grid's cell to another's of the same domain coordinates:
@@ -1886,7 +1907,8 @@ static int run_on_copies(const SweepSpec &sp, const Plan &pl, const uhs_params *
     const bool f64 = pl.st == kStF64, is2d = sp.rank == 2;
     const int R = pl.R;
     if (T < 4 || pl.kernel != UHS_KERNEL_STREAM || pl.cfg.k_temporal > 1 || pl.cfg.use_tma < 0 ||
-        (p && (p->flags & UHS_FLAG_IN_PLACE)) || (pl.shape == kBox3 && R >= 2) || !small_coordinates(sp))
+        (p && (p->flags & UHS_FLAG_IN_PLACE)) || (pl.shape == kBox3 && R >= 2) || !small_coordinates(sp) ||
+        outlives_thread(p, st))
         return UHS_OK;
     int64_t n[3], points = 1;
     for (int i = 0; i < 3; ++i) points *= n[i] = sp.ub[i] - sp.lb[i];
@@ -1982,9 +2004,9 @@ static int run_on_copies(const SweepSpec &sp, const Plan &pl, const uhs_params *
     if (!rc && !f64) rc = l_ab.launch();
     if (!rc) rc = l_b.launch();
     if (!rc) rc = l_a.launch();
-    if (f64) {
-        const int vrc = rc ? rc : waits(p) ? read_end(err, &run->state, st, end) : early.wait(end);
-        if (!rc) rc = vrc;
+    if (f64 && !rc) {
+        if (waits(p)) return read_end(err, &run->state, st, end, buf);
+        rc = early.wait(end);
     }
     cudaFreeAsync(buf, st);
     return rc;
@@ -1997,7 +2019,8 @@ static int run_on_copies(const SweepSpec &sp, const Plan &pl, const uhs_params *
 static int run_in_place_scanned(const SweepSpec &sp, const Plan &pl, const uhs_params *p, const GridView &va,
                                 const GridView &vb, int T, cudaStream_t st, bool *ran, RunEnd *end) {
     *ran = false;
-    if (!pl.auto_df32 || pl.kernel != UHS_KERNEL_STREAM || pl.cfg.k_temporal > 1 || !small_coordinates(sp))
+    if (!pl.auto_df32 || pl.kernel != UHS_KERNEL_STREAM || pl.cfg.k_temporal > 1 || !small_coordinates(sp) ||
+        outlives_thread(p, st))
         return UHS_OK;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) {
@@ -2030,7 +2053,10 @@ static int run_in_place_scanned(const SweepSpec &sp, const Plan &pl, const uhs_p
     if (e == cudaSuccess && !waits(p)) e = early.enqueue(&run->state, st);
     if (e != cudaSuccess) rc = cuda_error(e, "range scan");
     for (int t = 0; t < std::max(T, 1) && !rc; ++t) rc = (t % 2 ? ba : ab).launch();
-    if (!rc) rc = waits(p) ? read_end(err, &run->state, st, end) : early.wait(end);
+    if (!rc) {
+        if (waits(p)) return read_end(err, &run->state, st, end, buf);
+        rc = early.wait(end);
+    }
     cudaFreeAsync(buf, st);
     return rc;
 }
@@ -2290,7 +2316,7 @@ int uhs_sweep(const uhs_stencil_desc *d, const uhs_memref *in, const uhs_memref 
     RunEnd end;
     if ((rc = run_in_place_scanned(sp, pl, p, vi, vo, 1, st, &done, &end))) return rc;
     const bool native = end.state == kRunNative;
-    if (done && !native) return finish(p, st, &end);
+    if (done && !native) return finish_run(p, st, end, pl.auto_df32);
     if (pl.auto_df32 && (native || !range_ok(sp, vi, vo, 1, st, &pl.pair_shift))) {
         fall_back_native(pl);
     }
@@ -2320,7 +2346,7 @@ int uhs_run(const uhs_stencil_desc *d, const uhs_memref *a, const uhs_memref *b,
         (rc = run_in_place_scanned(sp, pl, p, va, vb, d->iterations, st, &done, &end)))
         return rc;
     const bool native = end.state == kRunNative;
-    if (done && !native) return finish(p, st, &end);
+    if (done && !native) return finish_run(p, st, end, pl.auto_df32);
     if (pl.auto_df32 && d->iterations > 0 &&
         (native || !range_ok(sp, va, vb, d->iterations, st, &pl.pair_shift))) {
         fall_back_native(pl);
