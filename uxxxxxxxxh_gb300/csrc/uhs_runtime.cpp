@@ -823,6 +823,8 @@ static int stream_zchunk(const SweepSpec &sp, const Plan &pl, const StreamCall &
                 }
             }
         }
+        // the launch grid's third axis holds 65535 chunks
+        zchunk = static_cast<int>(std::max<int64_t>(zchunk, (nz + 65534) / 65535));
     }
     if (occ_out) *occ_out = occ;
     return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(zchunk > 0 ? zchunk : 1, std::max<int64_t>(nz, 1))));
