@@ -188,13 +188,15 @@ int uhs_validate(const uhs_stencil_desc *desc, const uhs_memref *a, const uhs_me
  *
  * Resident runs: rank-2 star and box programs whose domain fits in the GPU's
  * shared memory (FP64 under UHS_ARITH_AUTO from two sweeps on, without
- * UHS_FLAG_NO_SYNC; FP32 from eight), with the launch left to the backend (params NULL or all zero apart
- * from flags, no tuner-database entry), run in one cooperative launch that
- * holds the grid on chip from the first sweep to the last and writes both
- * grids at its end.  Results are bit-identical to the sweeps launched one by
- * one.  Scratch: two words per cell from the library's pool; without it, on a
- * capturing stream, with UHS_FLAG_IN_PLACE, or on cudaStreamPerThread with
- * UHS_FLAG_NO_SYNC, the sweeps are launched one by one.  The kernel makes UHS_ARITH_AUTO's range check itself, over the cells
+ * UHS_FLAG_NO_SYNC; FP32 from eight), with the launch left to the backend
+ * (params NULL or all zero apart from flags, no tuner-database entry), run in
+ * one cooperative launch that holds the grid on chip from the first sweep to
+ * the last and writes both grids at its end.  Results are bit-identical to
+ * those of the sweeps launched one by one, on copies or in place as the next
+ * paragraph says.  Scratch: two words per cell from the library's pool;
+ * without it, on a capturing stream, with UHS_FLAG_IN_PLACE, or on
+ * cudaStreamPerThread with UHS_FLAG_NO_SYNC, the sweeps are launched one by
+ * one.  The kernel makes UHS_ARITH_AUTO's range check itself, over the cells
  * the program reads.
  *
  * Pair-resident runs: FP64 grids swept in float-pair arithmetic (UHS_ARITH_AUTO

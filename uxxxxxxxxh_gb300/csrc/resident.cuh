@@ -33,9 +33,9 @@
 //    pairs' power-of-two scale (pair_range); when the range needs native FP64
 //    it returns with both grids untouched and says so in *verdict.
 //  * Per point the sums are the streaming kernel's: the same terms, order and
-//    roundings, so results are bit-identical to it.  A program of fewer than
-//    8 sweeps rounds to FP64 between steps (round64), as the in-place sweeps
-//    it stands for do.
+//    roundings, so results are bit-identical to it.  A program whose sweeps
+//    would run in place (fewer than 8, or fewer than 4 from 2^21 points on)
+//    rounds to FP64 between steps (round64), as they do.
 //
 // Bound: instruction issue (float pairs) and latency in the walk, then the
 // exchange's round trip (about 1 us of the step).

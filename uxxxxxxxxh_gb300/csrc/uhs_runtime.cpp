@@ -1274,6 +1274,16 @@ static bool pair_eligible(const Plan &pl, int T, const uhs_params *p) {
            !(p && (p->flags & UHS_FLAG_IN_PLACE));
 }
 
+// Whether an FP64 run under UHS_ARITH_AUTO holds float pairs from step to step
+// (on copies, or on chip) or rounds to FP64 between them, as sweeps in place do:
+// one rule for every route, so that a flag or a stated launch parameter does not
+// change a result's last bits.  Copies pay from kPairMinT steps on; from
+// kSoloPoints points on, where the grid is out of L2 and an in-place sweep costs
+// a third more than a pair sweep, from four (8192^2 T = 4, 3d1r 512^3 T = 4).
+static bool pairs_between_steps(int T, int64_t points) {
+    return T >= kPairMinT || (T >= 4 && points >= kSoloPoints);
+}
+
 struct BatchSolo {
     SweepSpec sp;
     Plan pl;
@@ -1847,7 +1857,7 @@ static int run_resident(const SweepSpec &sp, const Plan &pl, const uhs_params *p
     c.L = rp.L;
     c.halo_off = rp.halo_off;
     c.T = T;
-    c.round64 = f64 && T < kPairMinT ? 1 : 0;
+    c.round64 = f64 && !pairs_between_steps(T, nz * nx) ? 1 : 0;
     c.growth = run_growth(sp, T);
     c.pub = buf;
     c.ctl = err + kRunCtlWord;
@@ -1890,11 +1900,9 @@ static GridView shifted_view(const GridView &g, const int64_t from[3], const int
 // 7.7; 3d1r star 200 x 200 x 201 38.3 / 24.5 -> 27 / 13; 3d1r star 512^3 364 /
 // 210 -> 337 / 176 (aligned lines).
 //
-// FP64 runs of T >= kPairMinT take copies as before; shorter ones (T >= 4) from
-// kSoloPoints points on, where the grid is out of L2 and an in-place sweep
-// costs a third more than a pair sweep (8192^2 T = 4, 3d1r 512^3 T = 4); below
-// that size they keep the in-place sweeps, whose results round to FP64 between
-// steps like the batched kernel's.  FP32 pays an extra sweep (step T - 1 goes
+// FP64 runs take copies where they hold pairs between steps
+// (pairs_between_steps); the others keep the in-place sweeps, whose results
+// round to FP64 between steps like the batched kernel's.  FP32 pays an extra sweep (step T - 1 goes
 // to the copy and to b) and the shell copy.  3D rows that TMA cannot load: us a
 // run, sweeps alone -> copies, 3d2r star T = 20: 64^2 x 65 145 -> 120, 100^2 x
 // 101 210 -> 165, 160^2 x 161 430 -> 271; T = 8: 81 -> 83, 113 -> 102; so from
@@ -1916,7 +1924,7 @@ static int run_on_copies(const SweepSpec &sp, const Plan &pl, const uhs_params *
     for (int i = 0; i < 3; ++i) points *= n[i] = sp.ub[i] - sp.lb[i];
     if (points <= 0) return UHS_OK;
     if (f64) {
-        if (!pl.auto_df32 || (T < kPairMinT && points < kSoloPoints)) return UHS_OK;
+        if (!pl.auto_df32 || !pairs_between_steps(T, points)) return UHS_OK;
     } else {
         if (pl.st != kStF32 || !params_are_auto(p) || (p && (p->flags & UHS_FLAG_XSHUFFLE))) return UHS_OK;
         StreamCall c = stream_call_of(sp, pl);
