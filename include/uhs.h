@@ -73,8 +73,7 @@ enum {
                             flushes to zero; 2^128 or more returns UHS_ERANGE).  Star
                             and separable sums run on an anchor set per point to twice
                             sum |c_k x_k| (anchored sums): each point's error stays within
-                            about n^2 2^-46 of that sum for n terms, and a point whose
-                            sum |c_k x_k| passes 2^126 returns UHS_ERANGE too */
+                            about n^2 2^-46 of that sum for n terms */
 };
 
 /* ---- MLIR memref descriptor (rank-3 layout) ---------------------------- */

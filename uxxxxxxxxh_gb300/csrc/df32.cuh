@@ -156,6 +156,17 @@ __device__ __forceinline__ u64 sub2(u64 a, u64 b) {
     return r;
 }
 
+__device__ __forceinline__ u64 mul2(u64 a, u64 b) {
+    u64 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c) {
+    u64 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
 // c * x of one point: the product's hi and its error with the cross terms
 // (as in df_mul / df_fma).
 __device__ __forceinline__ void df_prod(float ch, float cl, float2 x, float &p, float &e) {
@@ -225,8 +236,11 @@ namespace uhs {
 // sum |c| enters as 2 (1 + 2^-15) |ch| from the host (fill_coef_anchor), so
 // the anchor is one FMA per term and needs no further rounding.
 //
-// T reaches 3 B: a point whose B exceeds about 2^126.4 overflows to Inf/NaN,
-// which the range flag catches.
+// T reaches 3 B, which would overflow for points whose B lies between 2^126.4
+// and 2^128.  So the sums run on coefficients times 2^-2 (fill_coef_anchor) and
+// their results are multiplied by 4 (dfa_up, dfa_renorm_up): exact, and every
+// rounding the same but for low parts below 2^-124, which keep 2^-147.  It costs
+// one or two packed operations for two points.
 __device__ __forceinline__ float anchor_add(float b, float cabs, float2 x) {  // cabs = 2 (1 + 2^-15) |ch|
     return __fmaf_rn(cabs, fabsf(x.x), b);
 }
@@ -264,6 +278,14 @@ __device__ __forceinline__ df dfa_end(const dfa &a) {
 __device__ __forceinline__ float2 dfa_renorm(df a) {
     const float s = __fadd_rn(a.h, a.l);
     return make_float2(s, __fsub_rn(a.l, __fsub_rn(s, a.h)));
+}
+
+// the sum of the unscaled coefficients, and its renormalised pair: the four-fold
+// high part is fused into the two additions that dfa_renorm has
+__device__ __forceinline__ df dfa_up(df a) { return df{__fmul_rn(a.h, 4.0f), __fmul_rn(a.l, 4.0f)}; }
+__device__ __forceinline__ float2 dfa_renorm_up(df a) {
+    const float l = __fmul_rn(a.l, 4.0f), s = __fmaf_rn(a.h, 4.0f, l);
+    return make_float2(s, __fsub_rn(l, __fmaf_rn(a.h, -4.0f, s)));
 }
 
 // The same for two points at once: the subtractions and the hi additions
@@ -304,6 +326,15 @@ __device__ __forceinline__ df2 dfa2_end(const dfa2 &a) {
 __device__ __forceinline__ void dfa2_renorm(const df2 &a, u64 &h, u64 &l) {
     h = add2(a.h, a.l);
     l = sub2(a.l, sub2(h, a.h));
+}
+__device__ __forceinline__ df2 dfa2_up(const df2 &a) {
+    const u64 four = pk2(4.0f, 4.0f);
+    return df2{mul2(a.h, four), mul2(a.l, four)};
+}
+__device__ __forceinline__ void dfa2_renorm_up(const df2 &a, u64 &h, u64 &l) {
+    const u64 four = pk2(4.0f, 4.0f), l4 = mul2(a.l, four);
+    h = fma2(a.h, four, l4);
+    l = sub2(l4, fma2(a.h, pk2(-4.0f, -4.0f), h));
 }
 
 // acc += g, an (unnormalised) pair: TwoSum of the high parts.  Adds a group of

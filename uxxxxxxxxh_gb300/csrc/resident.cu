@@ -16,7 +16,7 @@ cudaError_t launch_cfg(const ResCall &c, int smem, const double *coef, cudaStrea
     args.c = c;
     double cd[NT];
     fill_coefs(cd, args.chl, args.cl_sum, coef, NT, SHAPE, R);
-    fill_coef_anchor(args.cab, args.chl, NT);
+    if (ST == kStF64) fill_coef_anchor(args.cab, args.chl, NT, SHAPE, R, false);
     auto kern = k_resident<SHAPE, R, ST>;
     // the largest size once per device, so concurrent launches never see a smaller one
     static std::atomic<bool> ready[64];

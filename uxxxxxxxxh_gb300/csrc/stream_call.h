@@ -16,7 +16,7 @@ constexpr bool is_rank2_shape(int shape) { return shape == kStar2 || shape == kB
 enum { kStF64 = 0, kStF32 = 1, kStF32x2 = 2 };
 enum { kArNative = 0, kArDf32 = 1 };
 enum { kLdCpAsync = 0, kLdTma = 1 };
-enum { kIoPlain = 0, kIoFirst = 1, kIoLast = 2 };
+enum { kIoPlain = 0, kIoFirst = 1, kIoLast = 2, kIoRun = 3 };
 // The range scan's verdict on an FP64 run (range_scan.cu), read by its kernels.
 enum { kRunPairs = 1, kRunNative = 2 };
 struct PairRun {
@@ -76,7 +76,29 @@ inline void fill_coefs(double *cd, float2 *chl, float *cl_sum, const double *coe
     }
     for (int i = 0; i < 3; ++i) cl_sum[i] = static_cast<float>(sums[i]);
 }
-inline void fill_coef_anchor(float *cab, const float2 *chl, int nt) {
+// Float-pair sums on an anchor (df32.cuh): stars, separable boxes and the columns
+// of term-by-term 3D boxes of radius 2-3.  They reach 3 sum |c x|, so they run on
+// coefficients times 2^-2 (kAnchorDown) and their results are multiplied back
+// (kAnchorUp): without it points whose sum |c x| lies between 2^126.4 and 2^128
+// overflowed.  Powers of two, so every rounding above the float range's lowest
+// binades is the same.  A separable box's first pass (x, the last slots) takes
+// the factor for all of its passes.  Runs whose range was scanned stay below
+// 2^120 and keep the coefficients as they are in the kernels that are theirs
+// alone (resident runs; kIoFirst, kIoRun, kIoLast).
+constexpr float kAnchorDown = 0.25f, kAnchorUp = 4.0f;
+__host__ __device__ constexpr bool is_anchored(int shape, int R) {
+    return shape == kStar3 || shape == kStar2 || shape == kSep3 || shape == kSep2 || (shape == kBox3 && R >= 2);
+}
+// chl of a float-pair sweep (scaled: with the factor), and 2 (1 + 2^-15) |ch|, its
+// anchors' operands
+inline void fill_coef_anchor(float *cab, float2 *chl, int nt, int shape, int R, bool scaled) {
+    if (scaled && is_anchored(shape, R)) {
+        const bool sep = shape == kSep3 || shape == kSep2;
+        for (int k = sep ? nt - (2 * R + 1) : 0; k < nt; ++k) {
+            chl[k].x *= kAnchorDown;
+            chl[k].y *= kAnchorDown;
+        }
+    }
     const float f = 2.0f * (1.0f + 0x1p-15f);
     for (int k = 0; k < nt; ++k) cab[k] = f * (chl[k].x < 0.0f ? -chl[k].x : chl[k].x);
 }
@@ -137,8 +159,9 @@ cudaError_t launch_stream_f64n_2d(const StreamCall &c);
 cudaError_t launch_stream_f64df_2d(const StreamCall &c);
 cudaError_t launch_stream_f32_2d(const StreamCall &c);
 cudaError_t launch_stream_f32x2_2d(const StreamCall &c);
-// First and last sweeps of runs on float-pair copies (kIoFirst, kIoLast): the
-// planner's default tiles, kIoLast by TMA (term-by-term 2D boxes: cp.async).
+// First, middle and last sweeps of runs on float-pair copies (kIoFirst, kIoRun,
+// kIoLast): the planner's default tiles, kIoRun and kIoLast by TMA (kIoLast of
+// term-by-term 2D boxes: cp.async; kIoRun: anchored sums only).
 cudaError_t launch_stream_ends_3d(const StreamCall &c);
 cudaError_t launch_stream_ends_2d(const StreamCall &c);
 

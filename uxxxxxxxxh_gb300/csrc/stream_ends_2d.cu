@@ -1,7 +1,7 @@
-// First and last sweeps of runs on float-pair copies of FP64 grids: the FP64
-// grid read and pairs written, and pairs read and the FP64 grid written, so
-// that a run needs no conversion passes.  One tile per shape, the planner's
-// default.
+// Sweeps of runs on float-pair copies of FP64 grids: the first reads the FP64
+// grid and writes pairs, the last ones read pairs and write the FP64 grid, so
+// that a run needs no conversion passes; the ones between them sum without the
+// anchored sums' factor.  One tile per shape, the planner's default.
 #include "stream_launch.cuh"
 
 namespace uhs {
@@ -12,6 +12,10 @@ namespace {
 template <int SHAPE, int R>
 cudaError_t dispatch(const StreamCall &c) {
     if constexpr (SHAPE == kStar2) {
+        if (c.io == kIoRun)
+            return c.ld == kLdTma && c.tile == 3
+                       ? launch_cfg<StreamCfg<SHAPE, R, kStF32x2, kArDf32, kLdTma, 64, 1, 1, 4, 0, 2, kIoRun>>(c)
+                       : cudaErrorInvalidValue;
         if (c.io == kIoLast)
             return c.ld == kLdTma && c.tile == 3
                        ? launch_cfg<StreamCfg<SHAPE, R, kStF32x2, kArDf32, kLdTma, 64, 1, 1, 4, 0, 2, kIoLast>>(c)
@@ -22,6 +26,12 @@ cudaError_t dispatch(const StreamCall &c) {
     } else {
         constexpr int LAST = SHAPE == kBox2 ? kLdCpAsync : kLdTma;
         if (c.tile != 0) return cudaErrorInvalidValue;
+        if (c.io == kIoRun) {
+            if constexpr (SHAPE == kSep2)
+                if (c.ld == kLdTma)
+                    return launch_cfg<StreamCfg<SHAPE, R, kStF32x2, kArDf32, kLdTma, 128, 1, 1, 4, 0, 1, kIoRun>>(c);
+            return cudaErrorInvalidValue;
+        }
         if (c.io == kIoLast)
             return c.ld == LAST ? launch_cfg<StreamCfg<SHAPE, R, kStF32x2, kArDf32, LAST, 128, 1, 1, 4, 0, 1, kIoLast>>(c)
                                 : cudaErrorInvalidValue;

@@ -1,7 +1,8 @@
-// First and last sweeps of runs on float-pair copies of FP64 grids: the FP64
-// grid read and pairs written, and pairs read and the FP64 grid written, so
-// that a run needs no conversion passes.  One tile per shape, the planner's
-// default.  Term-by-term boxes of radius 2-3 have none: their sums dwarf the
+// Sweeps of runs on float-pair copies of FP64 grids: the first reads the FP64
+// grid and writes pairs, the last ones read pairs and write the FP64 grid, so
+// that a run needs no conversion passes; the ones between them sum without the
+// anchored sums' factor.  One tile per shape, the planner's default.
+// Term-by-term boxes of radius 2-3 have none: their sums dwarf the
 // conversion passes.
 #include "stream_launch.cuh"
 
@@ -11,6 +12,11 @@ namespace {
 template <int SHAPE, int R>
 cudaError_t dispatch(const StreamCall &c) {
     constexpr int TY = 4, VY = 4, PD = 3;
+    if (c.io == kIoRun) {
+        if constexpr (is_anchored(SHAPE, R))
+            if (c.ld == kLdTma) return launch_cfg<StreamCfg<SHAPE, R, kStF32x2, kArDf32, kLdTma, 32, TY, VY, PD, 0, 1, kIoRun>>(c);
+        return cudaErrorInvalidValue;
+    }
     if (c.io == kIoLast)
         return c.ld == kLdTma ? launch_cfg<StreamCfg<SHAPE, R, kStF32x2, kArDf32, kLdTma, 32, TY, VY, PD, 0, 1, kIoLast>>(c)
                               : cudaErrorInvalidValue;

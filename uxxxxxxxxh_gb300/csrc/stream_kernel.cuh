@@ -79,7 +79,8 @@ __host__ __device__ constexpr int coef_slot(int dz, int dy, int dx) {
 // IO: what the sweep reads and writes.  kIoPlain: grids of one type.  The ends
 // of a run on float-pair copies: kIoFirst reads the FP64 grid and writes
 // pairs, kIoLast reads pairs and writes the FP64 grid (and, for step T - 1,
-// the pairs too, StreamArgs::out2).
+// the pairs too, StreamArgs::out2).  kIoRun: the sweeps between them, which are
+// kIoPlain without the anchored sums' factor (SCALED).
 template <int SHAPE_, int R_, int ST_, int AR_, int LD_, int BX_, int TYT_, int VY_, int PD_, int XS_ = 0,
           int VX_ = 1, int IO_ = kIoPlain>
 struct StreamCfg {
@@ -138,6 +139,11 @@ struct StreamCfg {
     // 1.8); not for 2D boxes or 27 terms of mixed signs (25 terms 1.3 -> 2.3,
     // 27 terms 1.34 -> 1.54), which keep it.
     static constexpr bool GROUPED = AR == kArDf32 && SHAPE == kBox3 && R >= 2;
+    // sums on an anchor: on coefficients times 2^-2, their results multiplied back
+    // (three registers in the 3D 13-point pair sweep, 4 CTAs an SM instead of 5:
+    // 10.53 -> 10.84 ms at 512^3, T = 20; other sweeps within 1 %.  So not in the
+    // kernels of scanned runs)
+    static constexpr bool SCALED = AR == kArDf32 && is_anchored(SHAPE, R) && IO == kIoPlain;
     static_assert(LD != kLdTma || W <= 256, "TMA boxes are at most 256 elements wide");
     static_assert(!SI::is2d || (TYT == 1 && VY == 1), "rank-2 tiles are one row");
     static_assert(!XS || (SI::is2d && SI::star), "lane shuffles: rank-2 stars");
@@ -353,35 +359,58 @@ struct Arith<C, kArDf32> {
     __device__ static __forceinline__ Acc send(const SAcc &acc) { return dfa_end(acc); }
     // sums of stars and separable passes end as dfa_end's pairs
     static constexpr bool kFastRenorm = C::SI::star || C::SI::sep;
-    __device__ static __forceinline__ float2 norm(const Acc &acc) {
+    // a pass's value between the passes of a separable box
+    __device__ static __forceinline__ float2 level(const Acc &acc) {
         if constexpr (kFastRenorm) return dfa_renorm(acc);
         else return renorm(acc);
+    }
+    // a point's result: the sum with the anchored sums' factor taken out
+    __device__ static __forceinline__ Acc up(const Acc &acc) {
+        if constexpr (C::SCALED) return dfa_up(acc);
+        else return acc;
+    }
+    __device__ static __forceinline__ float2 norm(const Acc &acc) {
+        if constexpr (kFastRenorm && C::SCALED) return dfa_renorm_up(acc);
+        else return C::SCALED ? renorm(up(acc)) : level(acc);
+    }
+    // the same for two points, packed
+    __device__ static __forceinline__ df2 up2(const df2 &acc) {
+        if constexpr (C::SCALED) return dfa2_up(acc);
+        else return acc;
+    }
+    __device__ static __forceinline__ void norm2(const df2 &acc, u64 &h, u64 &l) {
+        if constexpr (kFastRenorm && C::SCALED) dfa2_renorm_up(acc, h, l);
+        else if constexpr (kFastRenorm) dfa2_renorm(acc, h, l);
+        else renorm2(up2(acc), h, l);
     }
     // FP64 grids: joined back with the run's exponent bias (the pairs hold
     // x * 2^pair_shift).  A sum that outgrew the float range (hi Inf or NaN)
     // would join to a finite double; it sets the range flag instead of
     // passing unnoticed.
+    // (acc: up() already taken)
+    __device__ static __forceinline__ void join(double *p, const Acc &acc, unsigned &range_err, int bias) {
+        range_err |= (__float_as_uint(acc.h) & 0x7f800000u) == 0x7f800000u;
+        *p = join_f64(acc.h, acc.l, bias);
+    }
+    __device__ static __forceinline__ void join2(double *p, const Acc &a0, const Acc &a1, unsigned &range_err, int bias) {
+        range_err |= (__float_as_uint(a0.h) & 0x7f800000u) == 0x7f800000u;
+        range_err |= (__float_as_uint(a1.h) & 0x7f800000u) == 0x7f800000u;
+        *reinterpret_cast<double2 *>(p) = make_double2(join_f64(a0.h, a0.l, bias), join_f64(a1.h, a1.l, bias));
+    }
     __device__ static __forceinline__ void store(typename C::TO *p, const Acc &acc, unsigned &range_err, int bias) {
-        if constexpr (C::JOIN) {
-            range_err |= (__float_as_uint(acc.h) & 0x7f800000u) == 0x7f800000u;
-            *p = join_f64(acc.h, acc.l, bias);
-        } else {
-            *p = norm(acc);
-        }
+        if constexpr (C::JOIN) join(p, up(acc), range_err, bias);
+        else *p = norm(acc);
     }
     static constexpr bool kVecStore = true;
     __device__ static __forceinline__ void store2(typename C::TO *p, const Acc &a0, const Acc &a1, unsigned &range_err,
                                                   int bias) {
         if constexpr (C::JOIN) {
-            range_err |= (__float_as_uint(a0.h) & 0x7f800000u) == 0x7f800000u;
-            range_err |= (__float_as_uint(a1.h) & 0x7f800000u) == 0x7f800000u;
-            *reinterpret_cast<double2 *>(p) = make_double2(join_f64(a0.h, a0.l, bias), join_f64(a1.h, a1.l, bias));
+            join2(p, up(a0), up(a1), range_err, bias);
         } else {
             const float2 r0 = norm(a0), r1 = norm(a1);
             *reinterpret_cast<float4 *>(p) = make_float4(r0.x, r0.y, r1.x, r1.y);
         }
     }
-    __device__ static __forceinline__ float2 level(const Acc &acc) { return norm(acc); }
     template <class S, class Args>
     __device__ static __forceinline__ void centre(S &, const Args &, int, float2) {}
 };
@@ -927,8 +956,7 @@ __device__ __forceinline__ bool stream_item(const Args &a, int bxi, int byi, int
                     if constexpr (C::IO == kIoLast) {
                         if (optr2) {
                             u64 hh, ll;
-                            if constexpr (STAR || SEP) dfa2_renorm(acc[p], hh, ll);
-                            else renorm2(acc[p], hh, ll);
+                            A::norm2(acc[p], hh, ll);
                             upk2(hh, h0, h1);
                             upk2(ll, l0, l1);
                             if (2 * p >= vmin && 2 * p < vmax) optr2[2 * p * ostep2] = make_float2(h0, l0);
@@ -937,8 +965,7 @@ __device__ __forceinline__ bool stream_item(const Args &a, int bxi, int byi, int
                     }
                     if constexpr (C::OUT_PAIRS) {
                         u64 hh, ll;
-                        if constexpr (STAR || SEP) dfa2_renorm(acc[p], hh, ll);
-                        else renorm2(acc[p], hh, ll);
+                        A::norm2(acc[p], hh, ll);
                         upk2(hh, h0, h1);
                         upk2(ll, l0, l1);
                         if (VX == 2 && vmin == 0 && vmax == 2 && (reinterpret_cast<uintptr_t>(optr) & 15u) == 0) {
@@ -948,15 +975,16 @@ __device__ __forceinline__ bool stream_item(const Args &a, int bxi, int byi, int
                             if (2 * p + 1 < vmax) optr[(2 * p + 1) * ostep] = make_float2(h1, l1);
                         }
                     } else {
+                        acc[p] = A::up2(acc[p]);
                         upk2(acc[p].h, h0, h1);
                         upk2(acc[p].l, l0, l1);
                         if (VX == 2 && vmin == 0 && vmax == 2 && (reinterpret_cast<uintptr_t>(optr) & 15u) == 0) {
-                            A::store2(optr, df{h0, l0}, df{h1, l1}, range_err, bias);
+                            A::join2(optr, df{h0, l0}, df{h1, l1}, range_err, bias);
                         } else {
                             if (2 * p >= vmin && 2 * p < vmax)
-                                A::store(optr + 2 * p * ostep, df{h0, l0}, range_err, bias);
+                                A::join(optr + 2 * p * ostep, df{h0, l0}, range_err, bias);
                             if (2 * p + 1 < vmax)
-                                A::store(optr + (2 * p + 1) * ostep, df{h1, l1}, range_err, bias);
+                                A::join(optr + (2 * p + 1) * ostep, df{h1, l1}, range_err, bias);
                         }
                     }
                 }
@@ -1100,7 +1128,7 @@ __device__ __forceinline__ bool stream_item(const Args &a, int bxi, int byi, int
                 if (optr2) {
 #pragma unroll
                     for (int v = 0; v < NPT; ++v)
-                        if (v >= vmin && v < vmax) optr2[v * ostep2] = A::level(acc[v]);
+                        if (v >= vmin && v < vmax) optr2[v * ostep2] = A::norm(acc[v]);
                     optr2 += a.out2_s0;
                 }
             }

@@ -224,6 +224,7 @@ struct Plan {
     bool a_tmem = false;       // tensor-core path: A operand staged in tensor memory
     bool xshuffle = false;     // rank-2 stars: x-neighbours by warp shuffles
     const PairRun *run = nullptr;  // FP64 in float pairs decided on the device (launch_run_scan)
+    bool bounded = false;  // pair grids of a run whose range was scanned (pair_range): kIoRun
 };
 
 int device_sm_count() {
@@ -674,7 +675,10 @@ static bool make_tmap(const GridView &v, int eb, int W, int H, CUtensorMap *m) {
 
 static cudaError_t stream_dispatch(const StreamCall &c) {
     const bool is2d = is_rank2_shape(c.shape);
-    if (c.io != kIoPlain) return is2d ? launch_stream_ends_2d(c) : launch_stream_ends_3d(c);
+    // kIoRun: variants of the default launches of stars and separable boxes
+    const bool run = c.io == kIoRun && c.shape != kBox3 && c.shape != kBox2 && c.ld == kLdTma && !c.xshuffle &&
+                     c.tile == (!is2d ? 1 : c.shape == kStar2 ? 3 : 0);
+    if (c.io == kIoFirst || c.io == kIoLast || run) return is2d ? launch_stream_ends_2d(c) : launch_stream_ends_3d(c);
     if (c.st == kStF64 && c.ar == kArNative) return is2d ? launch_stream_f64n_2d(c) : launch_stream_f64n_3d(c);
     if (c.st == kStF64) return is2d ? launch_stream_f64df_2d(c) : launch_stream_f64df_3d(c);
     if (c.st == kStF32) return is2d ? launch_stream_f32_2d(c) : launch_stream_f32_3d(c);
@@ -876,7 +880,7 @@ static int prepare_stream(const SweepSpec &sp, const Plan &pl, const GridView &i
                           cudaStream_t st, unsigned *err_word, int io, StreamLaunch *l) {
     StreamCall &c = l->c;
     c = stream_call_of(sp, pl);
-    c.io = io;
+    c.io = io == kIoPlain && pl.bounded ? kIoRun : io;
     c.in = kernel_view(sp, in);
     c.out = kernel_view(sp, out);
     const bool is2d = sp.rank == 2;
@@ -1403,6 +1407,7 @@ static int batch_create(const uhs_stencil_desc *descs, const uhs_memref *as, con
                     q.arith = UHS_ARITH_DF32;
                     ErrorMessageGuard keep;
                     g.pairs = plan_sweep(g.sp2, &q, g.pa, &g.pl2) == UHS_OK && g.pl2.kernel == UHS_KERNEL_STREAM;
+                    g.pl2.bounded = pl.auto_df32;
                 } else {
                     cudaGetLastError();  // no copies: this grid sweeps in place
                 }
@@ -1982,6 +1987,7 @@ static int run_on_copies(const SweepSpec &sp, const Plan &pl, const uhs_params *
                 plan_sweep(sp, &ends, va, &first) == UHS_OK && first.kernel == UHS_KERNEL_STREAM &&
                 plan_sweep(sp2, &ends, pa, &last) == UHS_OK && last.kernel == UHS_KERNEL_STREAM;
         mid.run = first.run = last.run = run;
+        mid.bounded = f64;
         const GridView wb = shifted_view(vb, clb, sp.lb, cell), wa = shifted_view(va, clb, sp.lb, cell);
         ready = ready &&
                 prepare_stream(sp, first, va, shifted_view(pb, sp.lb, clb, cell), st, err, f64 ? kIoFirst : kIoPlain,
@@ -2074,8 +2080,8 @@ static int run_in_place_scanned(const SweepSpec &sp, const Plan &pl, const uhs_p
 // Pair-resident run of a float-pair FP64 program (see uhs_run in uhs.h):
 // *ran stays false when the scratch could not be had or planned, and the
 // caller then sweeps the FP64 grids in place.
-static int run_pair_resident(const SweepSpec &sp, const uhs_params *p, const GridView &va, const GridView &vb,
-                             int T, int shift, cudaStream_t st, bool *ran) {
+static int run_pair_resident(const SweepSpec &sp, const Plan &pl, const uhs_params *p, const GridView &va,
+                             const GridView &vb, int T, cudaStream_t st, bool *ran) {
     *ran = false;
     int dev = 0;
     cudaGetDevice(&dev);
@@ -2102,6 +2108,8 @@ static int run_pair_resident(const SweepSpec &sp, const uhs_params *p, const Gri
         ErrorMessageGuard keep;
         planned = plan_sweep(sp2, &q, pa, &pl2) == UHS_OK && pl2.kernel == UHS_KERNEL_STREAM;
     }
+    pl2.bounded = pl.auto_df32;
+    const int shift = pl.pair_shift;
     if (!planned) {
         cudaFreeAsync(buf, st);
         return UHS_OK;
@@ -2379,7 +2387,7 @@ int uhs_run(const uhs_stencil_desc *d, const uhs_memref *a, const uhs_memref *b,
     }
     if (pair_eligible(pl, d->iterations, p)) {
         bool ran = false;
-        rc = run_pair_resident(sp, p, va, vb, d->iterations, pl.pair_shift, st, &ran);
+        rc = run_pair_resident(sp, pl, p, va, vb, d->iterations, st, &ran);
         if (ran) return rc ? rc : finish(p, st);
     }
     if (d->iterations == 1) {
