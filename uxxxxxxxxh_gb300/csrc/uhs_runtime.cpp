@@ -1064,8 +1064,9 @@ static unsigned *pinned_end_words() {
 
 // A stream's status words, and the range verdict of an FP64 run (state, may be
 // NULL), once the stream has drained.  scratch (may be NULL, may hold the
-// verdict) is freed on the stream ahead of the wait, so that nothing of a call
-// that waits is pending when it returns.
+// verdict) is freed on the stream behind them: after the wait, which it would
+// lengthen by 2 us, except on cudaStreamPerThread, where nothing may be pending
+// when a call that waits returns (its thread may end).
 struct RunEnd {
     bool read = false;
     unsigned status[kStatusWords] = {};
@@ -1077,8 +1078,10 @@ static int read_end(const unsigned *w, const int *state, cudaStream_t st, RunEnd
     cudaError_t e = cudaMemcpyAsync(h, w, sizeof end->status, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess && state)
         e = cudaMemcpyAsync(h + kStatusWords, state, sizeof *state, cudaMemcpyDeviceToHost, st);
-    if (scratch) cudaFreeAsync(scratch, st);
+    const bool early = st == cudaStreamPerThread;
+    if (scratch && early) cudaFreeAsync(scratch, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (scratch && !early) cudaFreeAsync(scratch, st);
     if (e != cudaSuccess) return cuda_error(e, "device status read");
     std::memcpy(end->status, h, sizeof end->status);
     if (state) std::memcpy(&end->state, h + kStatusWords, sizeof end->state);
