@@ -66,7 +66,10 @@ struct ErrorMessageGuard {
     ~ErrorMessageGuard() { t_err = saved; }
 };
 
+// The thread's last CUDA error goes with the report: left behind, the next
+// call's first <<<>>> launch, which asks for it, would take it for its own.
 static int cuda_error(cudaError_t e, const char *what) {
+    cudaGetLastError();
     return set_error(UHS_ECUDA, "%s: %s (%s)", what, cudaGetErrorName(e), cudaGetErrorString(e));
 }
 
