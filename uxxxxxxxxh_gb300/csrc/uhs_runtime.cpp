@@ -1095,21 +1095,33 @@ static int read_end(const unsigned *w, const int *state, cudaStream_t st, RunEnd
 // The range verdict of a call that does not wait for its stream
 // (UHS_FLAG_NO_SYNC): copied right behind the scan, waited for alone while the
 // sweeps enqueued after it run on.
+// A call that fails before its wait waits all the same: the copy must not land
+// in words that a later call of the thread reads, or on a stack that is gone.
 struct EarlyVerdict {
     cudaEvent_t ev = nullptr;
+    cudaStream_t pending = nullptr;
+    bool copying = false, recorded = false;
     unsigned local = 0, *h = nullptr;
     ~EarlyVerdict() {
+        if (copying) recorded ? cudaEventSynchronize(ev) : cudaStreamSynchronize(pending);
         if (ev) cudaEventDestroy(ev);
     }
     cudaError_t enqueue(const int *state, cudaStream_t st) {
         h = pinned_end_words();
         if (!h) h = &local;
+        pending = st;
         cudaError_t e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(h, state, sizeof *h, cudaMemcpyDeviceToHost, st);
-        return e == cudaSuccess ? cudaEventRecord(ev, st) : e;
+        if (e == cudaSuccess) {
+            copying = true;
+            e = cudaMemcpyAsync(h, state, sizeof *h, cudaMemcpyDeviceToHost, st);
+        }
+        if (e == cudaSuccess) e = cudaEventRecord(ev, st);
+        recorded = e == cudaSuccess && copying;
+        return e;
     }
     int wait(RunEnd *end) {
         const cudaError_t e = cudaEventSynchronize(ev);
+        copying = false;
         if (e != cudaSuccess) return cuda_error(e, "range verdict");
         end->state = static_cast<int>(*h);
         return UHS_OK;
