@@ -42,6 +42,9 @@
 //
 // All waits are bounded (kResidentWaitCycles): one that runs out sets the
 // timeout flag, and every CTA returns.
+// Other streams' work delays a run but uses up none of its waits: a cooperative
+// launch starts when all of its CTAs can be placed (measured: beside a kernel that
+// held two SMs for 3 s, a run that needs every SM started at its end).
 #pragma once
 #include <type_traits>
 
