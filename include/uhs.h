@@ -213,9 +213,10 @@ int uhs_validate(const uhs_stencil_desc *desc, const uhs_memref *a, const uhs_me
  * returns it; the device's default pool is not touched).  When that
  * allocation fails, or with UHS_FLAG_IN_PLACE, the sweeps run on the FP64
  * grids directly, splitting on every load.  FP32 programs whose rows the
- * hardware cannot load in whole lines run on padded FP32 copies (8 bytes per
- * cell) in the same way, when the launch is left to the backend and the run is
- * long enough to pay for them.
+ * hardware cannot load in whole lines, and 3D radius-1 stars out of L2 (T >= 16
+ * on 2^24 points or more) whose rows do not start on 128-byte lines, run on
+ * padded FP32 copies (8 bytes per cell) in the same way, when the launch is left
+ * to the backend and the run is long enough to pay for them.
  *
  * Range: under UHS_ARITH_AUTO the pairs hold every value times 2^s, with s
  * chosen from a scan of the cells the program reads (a's domain and both

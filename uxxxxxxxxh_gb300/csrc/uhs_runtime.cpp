@@ -1898,6 +1898,12 @@ static int run_resident(const SweepSpec &sp, const Plan &pl, const uhs_params *p
     return UHS_OK;
 }
 
+// Whether every row of the domain starts on a 128-byte line.
+static bool rows_on_lines(const SweepSpec &sp, const GridView &g, int eb) {
+    const int64_t pitch = sp.rank == 3 ? g.s[0] | g.s[1] : g.s[1];
+    return (reinterpret_cast<uintptr_t>(g.data) + static_cast<uintptr_t>(sp.lb[2] * eb)) % 128 == 0 && pitch * eb % 128 == 0;
+}
+
 // Elements from one grid's cell to another's of the same domain coordinates:
 // out as seen by a kernel that indexes it with in's coordinates.
 static GridView shifted_view(const GridView &g, const int64_t from[3], const int64_t to[3], int eb) {
@@ -1932,7 +1938,7 @@ static GridView shifted_view(const GridView &g, const int64_t from[3], const int
 // 2^18 points at T >= 16, 2^20 at T >= 8.  Rows that TMA loads, or that 8-byte
 // cp.async pairs do for radius 1-2, only miss the lines: radius 1 out of L2
 // (512^3 T = 50 10.5 -> 9.3 ms; 3d1r at 129^2 x 130 T = 20 147 -> 163 us, 64^3
-// 87 -> 95).  2D rows that cannot load in 8-byte pairs: 3000 x 3001 21.9 -> 19.3
+// 87 -> 95; rows on lines already: sweeps alone).  2D rows that cannot load in 8-byte pairs: 3000 x 3001 21.9 -> 19.3
 // us a sweep.
 static int run_on_copies(const SweepSpec &sp, const Plan &pl, const uhs_params *p, const GridView &va,
                          const GridView &vb, int T, cudaStream_t st, bool *ran, RunEnd *end) {
@@ -1953,8 +1959,9 @@ static int run_on_copies(const SweepSpec &sp, const Plan &pl, const uhs_params *
         StreamCall c = stream_call_of(sp, pl);
         c.in = kernel_view(sp, va);
         const bool tma = pl.ld == kLdTma, in_pairs = rows_load_in_pairs(c, c.lb[2]);
+        const bool lined = rows_on_lines(sp, va, 4) && rows_on_lines(sp, vb, 4);
         if (is2d ? T < 16 || tma || in_pairs
-            : tma || (in_pairs && R <= 2) ? R > 1 || T < 16 || points < (int64_t(1) << 24)
+            : tma || (in_pairs && R <= 2) ? R > 1 || T < 16 || lined || points < (int64_t(1) << 24)
                                           : T < 8 || points < (int64_t(1) << (T < 16 ? 20 : 18)))
             return UHS_OK;
     }
