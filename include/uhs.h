@@ -370,7 +370,8 @@ int64_t uhs_launch_count(void);
 
 /* Return the device memory the library's scratch pools keep for reuse (the
  * float-pair copies of pair-resident runs) to the driver, on every device
- * used so far.  Memory of runs still in flight is released when they end. */
+ * used so far, and the pinned words that ended host threads left.  Memory of
+ * runs still in flight is released when they end. */
 int uhs_release_scratch(void);
 
 /* Diagnostics: exercise the failure-reporting path.  Launches one CTA whose

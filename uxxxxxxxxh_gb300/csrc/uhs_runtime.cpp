@@ -1047,18 +1047,41 @@ static int launch_fused_pass(const SweepSpec &sp, const Plan &pl, const GridView
 
 // Pinned words each host thread reads a stream's results into: the copies of
 // a call's end are enqueued together and waited for once (pageable copies are
-// staged and waited for one by one, 5-10 us each).  Freed with the thread.
+// staged and waited for one by one, 5-10 us each).  A thread that ends leaves
+// its words to the next one that asks (as many blocks as threads have called at
+// the same time; uhs_release_scratch gives the idle ones back).
 constexpr int kEndWords = kStatusWords + 1;
+struct PinnedPool {
+    std::mutex mu;
+    std::vector<unsigned *> idle;
+};
+static PinnedPool &pinned_pool() {
+    static PinnedPool *const pool = new PinnedPool;  // outlives every thread
+    return *pool;
+}
 static unsigned *pinned_end_words() {
     struct Words {
         unsigned *p = nullptr;
         ~Words() {
-            if (p) cudaFreeHost(p);
+            if (!p) return;
+            PinnedPool &pool = pinned_pool();
+            std::lock_guard<std::mutex> lk(pool.mu);
+            pool.idle.push_back(p);
         }
     };
     static thread_local Words w;
-    if (!w.p && cudaHostAlloc(reinterpret_cast<void **>(&w.p), kEndWords * sizeof(unsigned), cudaHostAllocPortable) !=
-                    cudaSuccess) {
+    if (w.p) return w.p;
+    PinnedPool &pool = pinned_pool();
+    {
+        std::lock_guard<std::mutex> lk(pool.mu);
+        if (!pool.idle.empty()) {
+            w.p = pool.idle.back();
+            pool.idle.pop_back();
+            return w.p;
+        }
+    }
+    if (cudaHostAlloc(reinterpret_cast<void **>(&w.p), kEndWords * sizeof(unsigned), cudaHostAllocPortable) !=
+        cudaSuccess) {
         cudaGetLastError();
         w.p = nullptr;
     }
@@ -1083,7 +1106,8 @@ static int read_end(const unsigned *w, const int *state, cudaStream_t st, RunEnd
         e = cudaMemcpyAsync(h + kStatusWords, state, sizeof *state, cudaMemcpyDeviceToHost, st);
     const bool early = st == cudaStreamPerThread;
     if (scratch && early) cudaFreeAsync(scratch, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    const cudaError_t drained = cudaStreamSynchronize(st);  // also where a copy was refused: another may be in flight
+    if (e == cudaSuccess) e = drained;
     if (scratch && !early) cudaFreeAsync(scratch, st);
     if (e != cudaSuccess) return cuda_error(e, "device status read");
     std::memcpy(end->status, h, sizeof end->status);
@@ -2174,6 +2198,12 @@ void uhs_params_default(uhs_params *p) {
 int64_t uhs_launch_count(void) { return g_launches.load(); }
 
 int uhs_release_scratch(void) {
+    {
+        PinnedPool &pool = pinned_pool();
+        std::lock_guard<std::mutex> lk(pool.mu);
+        for (unsigned *p : pool.idle) cudaFreeHost(p);
+        pool.idle.clear();
+    }
     std::lock_guard<std::mutex> lk(g_pool_mu);
     for (int dev = 0; dev < 64; ++dev) {
         if (!g_pools[dev]) continue;
