@@ -178,15 +178,34 @@ __global__ void __launch_bounds__(256) k_generic(const __grid_constant__ Generic
 
 // Points per thread (up to 4, in 2D 8): as many rows as the domain has for them, while the ring
 // leaves two CTAs an SM and the tiles, in chunks of 8 planes, still make two
-// CTAs for each SM.
-int generic_vy(const SweepSpec &sp, int TX, int TY, int eb) {
-    const int64_t nz = sp.ub[0] - sp.lb[0], ny = sp.ub[1] - sp.lb[1], nx = sp.ub[2] - sp.lb[2];
-    for (int vy = sp.rank == 2 ? 8 : 4; vy > 1; vy /= 2) {
+// CTAs for each SM.  FP64 programs gain less from more rows (a row costs an FP64
+// pipe term for each of its own, and a thread the time of one or two terms) than
+// the last tile's idle rows and, in 2D, an uneven last CTA an SM cost.  So of the
+// rows that rule allows they take those with the shortest estimate: 2D of the
+// busiest SM, 3D (whose chunks even the SMs out) of all rows, idle ones too.  us a
+// run, one row a thread / the most rows / these: 2D 49 points 217 x 2528 T = 8 518
+// / 776 / 518, 25 points EXACT 659 x 479 335 / 424 / 335, 5 points 4096^2 T = 2 460
+// / 372 / 372; 3D 125 points 152 x 37 x 213 T = 8 3080 / 3370 / 3080, 19 points 116 x
+// 77 x 257 915 / 1165 / 914, 7 points EXACT 182 x 156 x 128 978 / 817 / 820.
+int generic_vy(const SweepSpec &sp, int TX, int TY, int eb, bool exact) {
+    const int64_t nz = sp.ub[0] - sp.lb[0], ny = sp.ub[1] - sp.lb[1], nx = sp.ub[2] - sp.lb[2], sms = device_sm_count();
+    const auto tiles_y = [&](int vy) { return (ny + TY * vy - 1) / (TY * vy); };
+    int best = 1;
+    double shortest = 0.0;
+    for (int vy = sp.rank == 2 ? 8 : 4; vy >= 1; vy /= 2) {
         const size_t smem = static_cast<size_t>(2 * sp.rz + 2) * (TX + 2 * sp.rx) * (TY * vy + 2 * sp.ry) * eb;
-        const int64_t ctas = (nx + TX - 1) / TX * ((ny + TY * vy - 1) / (TY * vy)) * ((nz + 7) / 8);
-        if (smem <= 100 * 1024 && ctas >= 2 * device_sm_count()) return vy;
+        const int64_t ctas = (nx + TX - 1) / TX * tiles_y(vy) * ((nz + 7) / 8);
+        if (vy > 1 && (smem > 100 * 1024 || ctas < 2 * sms)) continue;
+        if (eb == 4) return vy;
+        const double terms = sp.nterms;
+        const double est = sp.rank == 3 ? static_cast<double>(tiles_y(vy)) * (vy + 2.0 / terms)
+                                        : static_cast<double>((ctas + sms - 1) / sms) * (vy + (exact ? 0.75 : 1.5) / terms);
+        if (shortest == 0.0 || est < shortest) {
+            shortest = est;
+            best = vy;
+        }
     }
-    return 1;
+    return best;
 }
 
 template <class T, int MAXT, bool EXACT, int VY>
@@ -263,7 +282,7 @@ cudaError_t launch_t(const SweepSpec &sp, const LaunchCfg &cfg, const GridView &
     for (int i = 0; i < 3; ++i)
         if (sp.ub[i] <= sp.lb[i]) return cudaSuccess;
     const int TX = cfg.tile_x > 0 ? cfg.tile_x : 32, TY = cfg.tile_y > 0 ? cfg.tile_y : 8;
-    switch (generic_vy(sp, TX, TY, sizeof(T))) {
+    switch (generic_vy(sp, TX, TY, sizeof(T), EXACT)) {
         case 8: return launch_v<T, MAXT, EXACT, 8>(sp, cfg, in, out, st);
         case 4: return launch_v<T, MAXT, EXACT, 4>(sp, cfg, in, out, st);
         case 2: return launch_v<T, MAXT, EXACT, 2>(sp, cfg, in, out, st);
