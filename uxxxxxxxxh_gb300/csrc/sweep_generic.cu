@@ -255,6 +255,23 @@ cudaError_t launch_v(const SweepSpec &sp, const LaunchCfg &cfg, const GridView &
         zchunk = (int)std::max<int64_t>(tiles * ((nz + least - 1) / least) < few ? 2 : least,
                                         (nz + want_chunks - 1) / want_chunks);
     }
+    if (sizeof(T) == 8 && VY > 1 && cfg.tile_z <= 0 && sp.rank == 3) {
+        // FP64 chunks that even the SMs out: several rows a thread make few CTAs an
+        // SM, and the busiest SM ends the sweep.  Up to twice the planes, where that
+        // leaves four CTAs an SM (below, they wait for latency and not for one
+        // another).  us a run, one row a thread / these rows in the usual chunks / in
+        // these: 7 points EXACT 160 x 247 x 195 T = 16 3822 / 4083 / 3856, 13 points 342 x
+        // 335 x 152 T = 8 3944 / 4068 / 3840.
+        const int64_t sms = device_sm_count();
+        const auto busiest = [&](int64_t zc) { return (tiles * ((nz + zc - 1) / zc) + sms - 1) / sms * (zc + 1); };
+        const int64_t z0 = zchunk;
+        int64_t best = busiest(z0) * 19 / 20;
+        for (int64_t z = z0 + 1; z <= 2 * z0 && tiles * ((nz + z - 1) / z) >= 4 * sms; ++z)
+            if (busiest(z) < best) {
+                best = busiest(z);
+                zchunk = static_cast<int>(z);
+            }
+    }
     a.zchunk = (int)std::min<int64_t>(zchunk, nz);
     const size_t smem = (size_t)a.NS * a.W * a.H * sizeof(T);
     auto kern = k_generic<T, MAXT, EXACT, VY>;
