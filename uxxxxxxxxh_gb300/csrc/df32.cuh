@@ -225,14 +225,15 @@ namespace uhs {
 // Why q is exact: at step k the terms before it took at most B - |p_k| from
 // the anchor, so T_{k-1} >= 2 B - (B - |p_k|) >= 2 |p_k| and T_k lies within
 // a factor of two of T_{k-1} (Sterbenz' lemma); the 2^-15 covers the
-// roundings of B and of the T's for up to 127 terms.  The same bound puts T_n
+// roundings of B and of the T's for the 3 to 19 terms that sums have here (and
+// well beyond).  The same bound puts T_n
 // between sigma / 2 and 2 sigma, so T_n - sigma is exact too.  All error is
 // in the three low-order accumulations: |r| <= ulp(3 B) / 2, and keeping the
 // r's apart from the cross terms (hi, lo) rounds each at its own size.
-// Measured on random sums of 5-19 terms (error / B, rms, in units of 2^-49):
-// 3.7-15 against 4.3-24 for the extraction on a power-of-two grid that was
-// used before (9 operations per term, one low-order accumulator), on every
-// count and sign pattern (tests/c/anchored_sum_check.c).
+// tests/c/anchored_sum_check.c holds the exact steps and the largest error of
+// random sums to these bounds on the host.  Compared once on random sums of 5-19
+// terms (error / B, rms, in units of 2^-49): 3.7-15 against 4.3-24 for an extraction
+// on a power-of-two grid (9 operations per term, one low-order accumulator).
 // sum |c| enters as 2 (1 + 2^-15) |ch| from the host (fill_coef_anchor), so
 // the anchor is one FMA per term and needs no further rounding.
 //

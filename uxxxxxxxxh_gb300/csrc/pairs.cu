@@ -1,14 +1,16 @@
-// FP64 grid <-> float-pair grid conversion for pair-resident runs.
+// FP64 grid <-> float-pair grid conversion for pair-resident runs that convert
+// in passes of their own: UHS_ARITH_DF32, term-by-term 3D boxes of radius 2-3, and
+// the large grids of batches.  (Other runs under UHS_ARITH_AUTO split in their
+// first sweep and join in their last ones, run_on_copies in uhs_runtime.cpp.)
 // The pairs may hold the values scaled by a power of two (df32.cuh): the
 // split applies the run's scale and the join removes it.
 //
 // A program of T >= 8 float-pair sweeps on FP64 grids (pair_eligible in
-// uhs_runtime.cpp) runs on float-pair
-// copies of its grids: each FP64 value is split once
-// (split_f64) into a {hi, lo} float pair, the T sweeps read and write pairs
-// (no split on every load, no join on every store: the sweep kernel's
-// float-pair variant), and the domain of each grid a sweep wrote is joined
-// back into the FP64 grid at the end.  Cells outside the domain (the halo)
+// uhs_runtime.cpp) runs on float-pair copies of its grids: each FP64 value is
+// split once (split_f64) into a {hi, lo} float pair, the T sweeps read and
+// write pairs (no split on every load, no join on every store: the sweep
+// kernel's float-pair variant), and the domain of each grid a sweep wrote is
+// joined back into the FP64 grid at the end.  Cells outside the domain (the halo)
 // are read from the FP64 grids' own values and never written back, so they
 // stay bit-exact.
 #include "df32.cuh"

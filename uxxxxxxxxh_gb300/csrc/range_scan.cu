@@ -1,10 +1,16 @@
 // Exponent range of FP64 grids, for choosing the arithmetic of an FP64
 // program: float pairs (df32) hold a value to 2^-48 of itself only between
-// 2^-74 and 2^128, so the planner runs df32 only when the largest magnitude,
+// 2^-74 and 2^128, so a program runs df32 only when the largest magnitude,
 // grown by (sum |c|)^T, stays well below 2^128 and the smallest nonzero
-// magnitude well above 2^-74.  Reads the grid's whole span (padding
-// included) once as 64-bit words and folds the biased exponent fields with
-// integer max and min; one atomicMax and one atomicMin per warp.
+// magnitude well above 2^-74 (pair_range).  Both kernels fold the biased
+// exponent fields with integer max and min.
+//   k_run_scan        the cells a run reads (a's domain, both grids' shells); its
+//                     verdict stays on the device, for the run's own kernels
+//   k_exponent_range  a grid's whole span (padding included) as 64-bit words, for
+//                     the host's choice: batches, temporal fusion, term-by-term 3D
+//                     boxes of radius 2-3 from 8 sweeps on, and calls without
+//                     scratch (one atomicMax and one atomicMin per warp)
+// and k_shell_copy fills the shells of a run's copies.
 #include "df32.cuh"
 #include "resident.h"
 #include "uhs_kernels.h"

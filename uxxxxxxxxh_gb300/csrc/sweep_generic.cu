@@ -25,7 +25,8 @@
 // 90-93 % of the measured DFMA rate); FP32 programs by instruction issue (79 %
 // of the slots).  us per sweep with one point per thread and coefficients
 // converted at each use -> now, 7-term one-sided program at 256^3: FP32 224 ->
-// 64, FP64 265 -> 248, EXACT 445 -> 445; 64^3 FP32 20 -> 11, FP64 21 -> 14;
+// 64, FP64 265 -> 248, EXACT 445 -> 445 (FP64 takes several rows only where they
+// pay, generic_vy); 64^3 FP32 20 -> 11, FP64 21 -> 14;
 // 5-term 2D at 4096^2: FP32 209 -> 58 (8 points a thread; 90 at 4), FP64 211 ->
 // 169.
 #include "uhs_kernels.h"

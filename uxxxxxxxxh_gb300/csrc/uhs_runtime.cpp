@@ -501,7 +501,7 @@ static int plan_sweep(const SweepSpec &sp, const uhs_params *p, const GridView &
         // slower).
         if (cfg.tile_x == 0 && p->vx == 0 && shape == kStar2 && !(p->flags & UHS_FLAG_XSHUFFLE)) {
             const bool tma = tma_aligned && cfg.use_tma >= 0;
-            // (FP64 grids swept in place, bounded sums, at 8192^2: 256 columns
+            // (FP64 grids swept in place, with 9-operation sums, at 8192^2: 256 columns
             // by cp.async 229 / 194 GStencil/s for r1 / r2 against 217 / 190
             // at 128 by TMA; radius 3 one point per thread, 129 vs 122)
             if (arith == UHS_ARITH_DF32) {
@@ -524,7 +524,7 @@ static int plan_sweep(const SweepSpec &sp, const uhs_params *p, const GridView &
             // 189 vs 191); 3d2r/3d3r stars 186/134 vs 181/127 at 64 x 8;
             // separable boxes r1/r2/r3 235/125/79 (FP64 in place 163/102/68)
             // vs 231/122/76 (162/98/60) at 32 x 32
-            // (with bounded sums FP64 grids swept in place prefer it too:
+            // (with 9-operation sums FP64 grids swept in place prefer it too:
             // 3d1r star 190 vs 177 GStencil/s at 64 x 8)
             if (shape == kStar3) tile = 1;
             else tile = 1;  // separable and term-by-term boxes (3d1r box 81.6 vs 75.9 at 32 x 32)
@@ -699,12 +699,18 @@ static GridView kernel_view(const SweepSpec &sp, const GridView &v) {
     return k;
 }
 
+// log2 of the largest factor T sweeps can grow a magnitude by, (sum |c|)^T
+// where that exceeds 1.
+static double run_growth(const SweepSpec &sp, int T) {
+    double csum = 0.0;
+    for (int k = 0; k < sp.nterms; ++k) csum += std::fabs(sp.coef[k]);
+    return csum > 1.0 ? std::max(T, 1) * std::log2(csum) : 0.0;
+}
 // UHS_ARITH_AUTO on FP64 grids.  A float pair holds a value to 2^-48 of
 // itself between 2^-74 and 2^128 (df32.cuh), and a run may keep every value
 // scaled by 2^s, which moves that window anywhere in the FP64 range (a linear
-// sweep commutes with the scale exactly).  Scan both grids (their whole
-// spans, halo included) for their exponent range and keep float pairs only
-// when
+// sweep commutes with the scale exactly).  Runs keep float pairs only when, in the
+// cells that are scanned,
 //   * no cell holds Inf or NaN;
 //   * with s chosen so that the largest magnitude grown by (sum |c|)^T over
 //     the run stays below 2^120 (8 binades under the float range), every
@@ -715,13 +721,10 @@ static GridView kernel_view(const SweepSpec &sp, const GridView &v) {
 // about 2^169 between its largest (grown) and smallest nonzero magnitudes is
 // the case left to native arithmetic: in float pairs its small cells would
 // keep 24 bits or flush to zero, which a max-normalised error would not show.
-// log2 of the largest factor T sweeps can grow a magnitude by, (sum |c|)^T
-// where that exceeds 1.
-static double run_growth(const SweepSpec &sp, int T) {
-    double csum = 0.0;
-    for (int k = 0; k < sp.nterms; ++k) csum += std::fabs(sp.coef[k]);
-    return csum > 1.0 ? std::max(T, 1) * std::log2(csum) : 0.0;
-}
+// The scan covers the cells the program reads where the device decides
+// (launch_run_scan, k_resident), and both grids' whole spans, halo included, here,
+// where the host does: batches, temporal fusion, term-by-term 3D boxes of radius 2-3
+// from 8 sweeps on, calls without scratch.
 static bool range_ok(const SweepSpec &sp, const GridView &a, const GridView &b, int T, cudaStream_t st,
                      int *shift) {
     *shift = 0;
